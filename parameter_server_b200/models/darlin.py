@@ -173,6 +173,9 @@ class DarlinSolver:
         self.seq = 0
         self.bar = 0
         self.kernel_launches = 0
+        # one GPU, resident matrix: 0 = the pass kernel runs on the whole GPU or in one thread-block cluster,
+        # whichever suits the non-zeros of a group of blocks; 1 / 2 = always the former / the latter
+        self.pass_variant = 0
 
     # ------------------------------------------------------------------ preprocessing
     def _drop_tail_features(self, offsets: torch.Tensor, keys: torch.Tensor, vals: Optional[torch.Tensor]):
@@ -502,8 +505,9 @@ class DarlinSolver:
                              self.local_bar.data_ptr(), self.bar, self.abort.data_ptr(), self.status.data_ptr(), None,
                              None if prev is None else prev.data_ptr(), 0 if prev is None else prev.numel(),
                              self.wide_block_cols, self.blk_gc.data_ptr(), self.blk_gs0.data_ptr(),
-                             1 if self.gather_small_groups else 0, 0, self.phase_ns.data_ptr(),
-                             None if self._all_cb is None else self._all_cb.data_ptr(), self.nblk, self.list_block_cols)
+                             1 if self.gather_small_groups else 0, self.pass_variant, self.phase_ns.data_ptr(),
+                             None if self._all_cb is None else self._all_cb.data_ptr(), self.nblk, self.list_block_cols,
+                             self.nnz * group // max(self.nblk, 1))
 
     def _build_structs(self):
         Wk = N.DarlinWorker(self.col_ptr.data_ptr(), self.row_idx.data_ptr(),

@@ -89,6 +89,60 @@ def test_bounded_delay_groups_match_oracle(tau):
     sol.check_status()
 
 
+@pytest.mark.parametrize("binary", [False, True])
+@pytest.mark.parametrize("rows,nnz,ratio,tau,wide", [
+    (40, 3, 2.0, 0, 0),          # blocks of a few non-zeros, some of a single chunk
+    (1500, 16, 1.0, 0, 0),
+    (9000, 40, 0.1, 0, 0),       # 90 k non-zeros per block: more than a cluster's threads keep in registers
+    (9000, 40, 0.2, 2, 0),       # the same over a bounded-delay group whose order ends in a shorter group
+    (9000, 40, 0.2, 2, 1),       # ... with every column stepped once in a phase of its own
+])
+@pytest.mark.parametrize("variant", [1, 2])
+def test_one_gpu_pass_variants_match_oracle(variant, rows, nnz, ratio, tau, wide, binary):
+    """The whole-GPU and the one-cluster form of the resident one-GPU pass."""
+    from parameter_server_b200.models.darlin import DarlinConfig, DarlinSolver
+    from parameter_server_b200.parallel.peer import PeerGroup
+
+    off, keys, vals, y = _problem(binary, rows=rows, nnz=nnz)
+    kw = dict(lambda1=0.3, max_pass=3, feature_block_ratio=ratio, seed=3, max_block_delay=tau)
+    sol = DarlinSolver(PeerGroup.single(torch.device("cuda", 0)), DarlinConfig(**kw), wide_block_cols=wide)
+    sol.pass_variant = variant
+    sol.preprocess(off, keys, vals, y)
+    prog = sol.run()
+    sol.check_status()
+    ref = DarlinRef([(off.cpu().numpy(), keys.cpu().numpy().view(np.uint64), None if vals is None else vals.cpu().numpy(),
+                      y.cpu().numpy())], None, RefConfig(**kw))
+    for p, r in zip(prog, ref.run()):
+        assert p.objv == pytest.approx(r.objv, rel=2e-3)
+        assert abs(p.nnz_w - r.nnz_w) <= max(3, 0.03 * r.nnz_w)
+        assert p.violation == pytest.approx(r.violation, rel=2e-2, abs=1e-3)
+    # the margins that were kept up to date are those of the weights
+    from parameter_server_b200.models.darlin import margins_from_weights
+    want = margins_from_weights(sol.col_ptr, sol.row_idx, sol.vals, sol.y, sol.w)
+    assert torch.allclose(sol.margin, want, rtol=1e-4, atol=1e-4)
+    assert torch.equal(sol.srv_gu.local[0], torch.zeros_like(sol.srv_gu.local[0]))
+
+
+@pytest.mark.parametrize("variant", [1, 2])
+def test_block_swept_twice_in_a_row_sees_its_own_update(variant):
+    """A block that follows itself in the order reads the columns that were written just before."""
+    from parameter_server_b200.models.darlin import DarlinConfig, DarlinSolver
+    from parameter_server_b200.parallel.peer import PeerGroup
+
+    off, keys, vals, y = _problem(False)
+    got = []
+    for orders in ([[0, 0, 1, 1, 1, 0]], [[0], [0], [1], [1], [1], [0]]):
+        sol = DarlinSolver(PeerGroup.single(torch.device("cuda", 0)), DarlinConfig(lambda1=0.3, feature_block_ratio=0.5, seed=3))
+        sol.pass_variant = variant
+        sol.preprocess(off, keys, vals, y)
+        for o in orders:
+            sol.launch_pass(np.asarray(o, dtype=np.int32))
+        sol.check_status()
+        got.append((sol.w.clone(), sol.margin.clone(), sol.delta.clone()))
+    for a, b in zip(*got):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-5)      # sums of the same terms in another order
+
+
 def test_tail_feature_filter_drops_rare_columns():
     """Columns whose count-min estimate is <= tail_feature_freq are removed before training; the rest of the
     run equals the oracle on the data filtered by a NumPy restatement of the same sketch."""
