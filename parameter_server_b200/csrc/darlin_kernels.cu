@@ -930,8 +930,8 @@ darlin_pass_kernel(DarlinWorker Wk, DarlinPeers P, DarlinServer S, DarlinSched Q
 //   * kCluster: when a group has so few non-zeros that one thread-block cluster covers them, the whole pass
 //     runs in ONE cluster and the barriers are the hardware's cluster barrier.
 // Bound by those round trips and the barriers, not by bandwidth.  One pass on B200, darlin_pass_kernel -> this one:
-// 20,242 rows x 75 non-zeros, 300 blocks (5 k non-zeros each): 3.01 -> 1.38 ms (cluster); 677,399 rows, 300 blocks
-// (169 k each): 5.20 -> 2.96 ms; 100,000 rows x 120, 64 wide blocks in groups of 9 (1.7 M each): 0.87 -> 0.385 ms.
+// 20,242 rows x 75 non-zeros, 300 blocks (5 k non-zeros each): 3.01 -> 1.08 ms (cluster); 677,399 rows, 300 blocks
+// (169 k each): 5.20 -> 2.75 ms; 100,000 rows x 120, 64 wide blocks in groups of 9 (1.7 M each): 0.87 -> 0.38 ms.
 constexpr int kSoloThreads = 1024;
 constexpr int kSoloItems = 2;
 
@@ -1117,8 +1117,11 @@ darlin_solo_kernel(DarlinWorker Wk, DarlinPeers P, DarlinServer S, DarlinSched Q
   __shared__ uint32_t s_abort;
   __shared__ SoloMeta s_meta[kMetaSlots];
   __shared__ uint64_t s_ns[4];
-  const int tid = (int)(blockIdx.x * blockDim.x + threadIdx.x), nthreads = (int)(gridDim.x * blockDim.x);
-  const int lane = threadIdx.x & 31, gwarp = tid >> 5, nwarps = nthreads >> 5;
+  // warps are numbered across the thread blocks: a group that gives work to only some warps, or a second round to
+  // some, gives every SM its share (numbered block by block: 1.38 instead of 1.08 ms, 2.96 instead of 2.75 ms)
+  const int nthreads = (int)(gridDim.x * blockDim.x), nwarps = nthreads >> 5;
+  const int lane = threadIdx.x & 31, gwarp = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+  const int tid = (nwarps - 1 - gwarp) * 32 + lane;     // the thread's number for columns: the idle warps' first
   const int group = min(Q.group > 0 ? Q.group : 1, kMetaSlots / 4);
   const int64_t wide_cols = min(Q.wide_cols > 0 ? (int64_t)Q.wide_cols : kWideBlockCols, (int64_t)nthreads);
   float* srv_w = P.w[P.rank];
@@ -1370,10 +1373,10 @@ using namespace psb;
 namespace {
 int g_darlin_grid[16] = {0};
 
-// Groups of blocks with at most this many non-zeros run in one cluster (16 blocks of 1024 threads, two non-zeros a
-// thread).  A pass of 300 groups: 5 k non-zeros a group 1.38 ms in a cluster, 1.55 ms on the whole GPU; 169 k a group
-// 8.5 ms against 2.96 ms.
-constexpr int64_t kSoloClusterNnz = 32768;
+// Groups of blocks with at most this many non-zeros run in one cluster of 16 blocks of 1024 threads.  Time per group,
+// cluster / whole GPU: 5 k non-zeros 3.6 / 4.3 us, 10 k 4.3 / 4.6, 20 k 5.7 / 5.2, 40 k 7.9 / 5.5, 169 k 27 / 9.2.
+// (A cluster of 8: 4.1 us at 5 k.)
+constexpr int64_t kSoloClusterNnz = 14336;
 
 struct SoloPlan { int sms = 0, cluster = 0; };
 

@@ -142,9 +142,9 @@ class DarlinSolver:
         reference's ``FeatureStation`` in ``-mmap_training_data`` mode with its task-id keyed look-ahead
         prefetch (src/linear_method/feature_station.cc:212-279, src/linear_method/darling.cc:175-201)."""
         self.group, self.cfg, self.impl = group, cfg, impl
-        # thread blocks of the pass kernel per SM (1 or 2): more blocks hide gather latency, fewer make the
-        # per-group barriers cheaper; 2 measured best with and without bounded delay (5.1 against 5.8 ms per
-        # pass on 677,399 x 47,236, one GPU)
+        # thread blocks of the pass kernel per SM (1 or 2) on several GPUs and out of core: more blocks hide gather
+        # latency, fewer make the per-group barriers cheaper; 2 measured best with and without bounded delay.  (One
+        # GPU with the matrix resident has a kernel that sizes its own grid.)
         self.ctas_per_sm = ctas_per_sm
         # groups of blocks with more local columns than this fetch the owners' sums once per column instead of
         # once per non-zero, at the price of one more in-GPU barrier (0: the kernel's default, 16384)
