@@ -34,7 +34,7 @@
 // block loop.
 #include <cstdlib>
 
-#include "psb_common.cuh"
+#include "reduce_kernels.cuh"
 
 namespace psb {
 
@@ -1292,6 +1292,51 @@ darlin_solo_kernel(DarlinWorker Wk, DarlinPeers P, DarlinServer S, DarlinSched Q
 #undef PSB_SOLO_TIME
 }
 
+// ---- what a rank reports after a pass, in one launch and one small copy to the host: loss of the margins, |w| and
+// non-zeros of the shard, its active set, the maximal KKT violation and the status word.  Terms and fp64 sums of
+// reduce_kernels.cuh, partial sums added in block order.  A pass over a small data set takes about a millisecond,
+// and the separate reductions, their copies and four synchronising reads took 0.2 ms more.
+constexpr int kProgressSums = 4;
+__global__ void __launch_bounds__(kReduceThreads)
+darlin_progress_kernel(const float2* __restrict__ ym, int64_t rows, const float* __restrict__ w, const uint8_t* __restrict__ active,
+                       int64_t slots, const float* __restrict__ violation, const uint32_t* __restrict__ status,
+                       double* partial /*[kProgressSums][kReduceMaxBlocks]*/, unsigned* ticket, double* out /*[8]*/) {
+  __shared__ double smem[kReduceThreads / 32];
+  __shared__ bool last;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  double s[kProgressSums] = {0.0, 0.0, 0.0, 0.0};
+  for (int64_t i = t0; i < rows; i += step) s[0] += reduce_term(kSumLogistic, ym[i].y);
+  for (int64_t i = t0; i < slots; i += step) {
+    s[1] += reduce_term(kSumAbs, w[i]);
+    s[2] += reduce_term(kCountNonZero, w[i]);
+    s[3] += (double)active[i];
+  }
+#pragma unroll
+  for (int k = 0; k < kProgressSums; ++k) {
+    const double v = block_sum_d(s[k], smem);
+    if (threadIdx.x == 0) partial[k * kReduceMaxBlocks + blockIdx.x] = v;
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < kProgressSums; ++k) {
+    double t = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) t += __ldcg(partial + k * kReduceMaxBlocks + b);
+    t = block_sum_d(t, smem);
+    if (threadIdx.x == 0) out[k] = t;
+  }
+  if (threadIdx.x == 0) {
+    out[4] = (double)*violation;
+    for (int k = 0; k < 3; ++k) out[5 + k] = (double)status[k];
+    *ticket = 0u;
+  }
+}
+
 // ---- stand-alone phase kernels (unfused NCCL baseline; gradients go to local buffers)
 __global__ void k_darlin_grad_local(DarlinWorker Wk, int64_t lc0, int64_t lc1, float2* gu_local) {
   // same reduction as phase A, accumulated into a local per-column buffer (index j − lc0)
@@ -1444,6 +1489,21 @@ int psb_darlin_pass(const DarlinWorker* Wk, const DarlinPeers* P, const DarlinSe
   DarlinWorker w = *Wk; DarlinPeers p = *P; DarlinServer s = *S; DarlinSched q = *Q; DarlinHyper h = *H;
   void* args[] = {&w, &p, &s, &q, &h};
   return (int)cudaLaunchCooperativeKernel((void*)darlin_pass_kernel, dim3(grid), dim3(512), args, 0, stream);
+}
+
+// scratch: psb_darlin_progress_scratch() bytes, zero before the first call; out: 8 device doubles
+// {loss, |w|, non-zero w, active, violation, status[0..2]}
+size_t psb_darlin_progress_scratch() { return (size_t)kProgressSums * kReduceMaxBlocks * 8 + 256; }
+int psb_darlin_progress(const void* ym, int64_t rows, const float* w, const uint8_t* active, int64_t slots, const float* violation,
+                        const uint32_t* status, void* scratch, double* out, cudaStream_t stream) {
+  double* partial = static_cast<double*>(scratch);
+  unsigned* ticket = reinterpret_cast<unsigned*>(partial + kProgressSums * kReduceMaxBlocks);
+  const int64_t n = rows > slots ? rows : slots;
+  int64_t grid = (n + kReduceThreads * 2 - 1) / (kReduceThreads * 2);
+  grid = grid < 1 ? 1 : grid > kReduceMaxBlocks ? kReduceMaxBlocks : grid;
+  darlin_progress_kernel<<<(int)grid, kReduceThreads, 0, stream>>>(static_cast<const float2*>(ym), rows, w, active, slots, violation,
+                                                                 status, partial, ticket, out);
+  return (int)cudaGetLastError();
 }
 
 // ---- out-of-core pass: the role of FeatureStation's prefetch threads

@@ -690,6 +690,21 @@ class DarlinSolver:
 
     def evaluate(self) -> tuple:
         """(objective, nnz_w, nnz_active, violation) summed/maxed over ranks (Darling::evaluateProgress)."""
+        return self._evaluate()[0]
+
+    def _evaluate(self):
+        """:meth:`evaluate` and the status word; one GPU reads both from the device with one copy."""
+        if self.group.world == 1 and self.impl == "fused":
+            if getattr(self, "_progress_scratch", None) is None:
+                self._lib.psb_darlin_progress_scratch.restype = C.c_size_t
+                self._progress_scratch = torch.zeros(self._lib.psb_darlin_progress_scratch(), dtype=torch.uint8, device=self.dev)
+                self._progress_out = torch.zeros(8, dtype=torch.float64, device=self.dev)
+            N.check(self._lib.psb_darlin_progress(N.ptr(self.ym), C.c_int64(self.rows), N.ptr(self.srv_w.local), N.ptr(self.srv_active),
+                                                  C.c_int64(self.slots), N.ptr(self.violation), N.ptr(self.status),
+                                                  N.ptr(self._progress_scratch), N.ptr(self._progress_out), N.stream_ptr()),
+                    "darlin_progress")
+            v = self._progress_out.tolist()
+            return (v[0] + self.cfg.lambda1 * v[1], int(v[2]), int(v[3]), v[4]), [int(x) for x in v[5:8]]
         loss = reduce_sum(self.margin.contiguous(), "sum_logistic")
         srv = self.srv_w.local[: max(self.slots, 0)]
         if self.slots > 0:
@@ -714,10 +729,12 @@ class DarlinSolver:
             dist.all_reduce(vals, group=self.group.group)
             dist.all_reduce(vio, op=dist.ReduceOp.MAX, group=self.group.group)
         v = vals.tolist()
-        return v[0] + self.cfg.lambda1 * v[1], int(v[2]), int(v[3]), float(vio.item())
+        return (v[0] + self.cfg.lambda1 * v[1], int(v[2]), int(v[3]), float(vio.item())), self.status.tolist()
 
     def check_status(self) -> None:
-        st = self.status.tolist()
+        self._raise_status(self.status.tolist())
+
+    def _raise_status(self, st) -> None:
         if st[0] != 0:
             raise RuntimeError(f"rank {self.group.rank}: {N.STATUS_NAMES.get(st[0], st[0])} (block={st[1]}, phase={st[2]})")
 
@@ -741,8 +758,8 @@ class DarlinSolver:
             else:
                 self.launch_pass(order, first=not prior)
         with nvtx_range("evaluate_progress"):
-            objv, nnz_w, nnz_as, vio = self.evaluate()
-        self.check_status()
+            (objv, nnz_w, nnz_as, vio), st = self._evaluate()
+        self._raise_status(st)
         if metrics is not None and self.group.rank == 0:
             metrics.log(event="pass", it=len(self.progress), objective=objv, nnz_w=nnz_w, active=nnz_as, violation=vio,
                         seconds=time.time() - t0, examples_per_s=self.total_rows / max(time.time() - t0, 1e-9),
