@@ -278,17 +278,16 @@ class DarlinSolver:
         if self.cfg.tail_feature_freq > 0:
             offsets, keys, vals = self._drop_tail_features(offsets, keys, vals)
         rows, nnz = y.numel(), keys.numel()
-        # unique local keys in unsigned order + column id of every non-zero  (Localizer::countUniqIndex/remapIndex)
-        lkeys, _ = sparse.count_unique(keys.contiguous())          # radix sort + run-length unique (unsigned order)
+        # unique local keys in unsigned order, the matrix by columns over them, the column of every non-zero (which
+        # saves the passes a column search per non-zero; not kept in out-of-core mode, where it would add 50 % to the
+        # bytes streamed from the host)
+        lkeys, col_ptr, row_idx, cvals, self.col_of = sparse.columns_from_rows(offsets, keys, vals, not self.out_of_core)
         uk = _ukey(lkeys)                                          # same keys as int64 values in that order
         P = lkeys.numel()
-        inv = sparse.remap(keys.contiguous(), lkeys)               # local column id of every non-zero
-        col_ptr, row_idx, cvals = sparse.csr_to_csc(offsets, inv, vals, P)   # CSR → CSC (SparseMatrix::alterStorage)
         # global statistics (ExampleInfo merge): rows, nnz, key range
         stats = g.all_reduce_sum([rows, nnz])
         self.total_rows, self.total_nnz = int(stats[0]), int(stats[1])
-        kmin = int(uk.min().item()) if P else (1 << 62)
-        kmax = int(uk.max().item()) if P else -(1 << 62)
+        kmin, kmax = torch.stack([uk[0], uk[-1]]).tolist() if P else (1 << 62, -(1 << 62))
         if W > 1:
             tmin = torch.tensor([kmin], dtype=torch.int64, device=dev)
             tmax = torch.tensor([kmax], dtype=torch.int64, device=dev)
@@ -369,10 +368,6 @@ class DarlinSolver:
         # label and margin of a row share 8 bytes: every non-zero gathers them with one access
         self.ym = torch.stack([y.to(f32), torch.zeros(rows, dtype=f32, device=dev)], 1).contiguous()
         self.margin = self.ym[:, 1]
-        # column id of every non-zero (saves a column search per non-zero and phase); not kept in out-of-core
-        # mode, where it would add 50 % to the bytes streamed from the host
-        self.col_of = None if self.out_of_core else torch.repeat_interleave(
-            torch.arange(P, dtype=torch.int32, device=dev), col_ptr[1:] - col_ptr[:-1]).contiguous()
         self.w = torch.zeros(P, dtype=f32, device=dev)
         self.delta = torch.full((P,), self.cfg.delta_init, dtype=f32, device=dev)
         self.active = torch.ones(P, dtype=torch.uint8, device=dev)

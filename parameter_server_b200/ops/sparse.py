@@ -25,6 +25,7 @@ def _lib():
         _L = N.lib()
         _L.psb_sort_tile.restype = C.c_size_t
         _L.psb_scan_tile.restype = C.c_size_t
+        _L.psb_column_tile.restype = C.c_size_t
     return _L
 
 
@@ -134,6 +135,45 @@ def csr_to_csc(offsets: torch.Tensor, col: torch.Tensor, vals: Optional[torch.Te
         out_vals = torch.empty(nnz, dtype=vals.dtype, device=dev)
         out_vals[dest[keep]] = vals[keep]
     return col_ptr, row_idx, out_vals
+
+
+def columns_from_rows(offsets: torch.Tensor, keys: torch.Tensor, vals: Optional[torch.Tensor], want_col_of: bool = True):
+    """CSR rows over uint64 keys → column-major storage over the unique keys, with one stable sort of the non-zeros:
+    (unique keys in unsigned order, col_ptr int64, row_idx int32, vals, column of every non-zero int32 or None).
+    ``Localizer::countUniqIndex`` + ``remapIndex`` + ``SparseMatrix::alterStorage``; the rows of a column ascend."""
+    lib, n, dev, rows = _lib(), keys.numel(), keys.device, offsets.numel() - 1
+    keys, offsets = keys.contiguous(), offsets.to(torch.int64).contiguous()
+    if n == 0 or n >= 1 << 32 or (vals is not None and vals.dtype != torch.float32):   # positions travel as 32-bit payloads
+        lkeys, _ = count_unique(keys)
+        col_ptr, row_idx, cvals = csr_to_csc(offsets, remap(keys, lkeys), vals, lkeys.numel())
+        col_of = torch.repeat_interleave(torch.arange(lkeys.numel(), dtype=torch.int32, device=dev),
+                                         col_ptr[1:] - col_ptr[:-1]) if want_col_of else None
+        return lkeys, col_ptr, row_idx, cvals, col_of
+    s = N.stream_ptr()
+    row_of = torch.empty(n, dtype=torch.int32, device=dev)
+    N.check(lib.psb_row_ids(N.ptr(offsets), C.c_int64(rows), _sz(n), N.ptr(row_of), s), "row_ids")
+    payload = row_of
+    if vals is not None:
+        vals = vals.contiguous()
+        payload = torch.empty(n, dtype=torch.int32, device=dev)
+        N.check(lib.psb_iota_u32(N.ptr(payload), _sz(n), s), "iota")
+    skeys, payload = sort_pairs(keys, payload)
+    tiles = torch.empty((n + lib.psb_column_tile() - 1) // lib.psb_column_tile(), dtype=torch.int64, device=dev)
+    total = torch.empty(1, dtype=torch.int64, device=dev)
+    N.check(lib.psb_column_heads(N.ptr(skeys), _sz(n), N.ptr(tiles), N.ptr(total), s), "column_heads")
+    lens = offsets[1:] - offsets[:-1]
+    ncols, nnz, shortest = torch.stack([total[0], lens.sum(), lens.min() if rows else total[0]]).tolist()
+    if nnz != n or shortest < 0:
+        raise ValueError(f"row offsets describe {nnz} non-zeros, there are {n}" if nnz != n else "row offsets must not decrease")
+    lkeys = torch.empty(ncols, dtype=torch.int64, device=dev)
+    col_ptr = torch.empty(ncols + 1, dtype=torch.int64, device=dev)
+    row_idx = torch.empty(n, dtype=torch.int32, device=dev)
+    cvals = None if vals is None else torch.empty(n, dtype=torch.float32, device=dev)
+    col_of = torch.empty(n, dtype=torch.int32, device=dev) if want_col_of else None
+    N.check(lib.psb_column_write(N.ptr(skeys), N.ptr(payload), _sz(n), _sz(ncols), N.ptr(tiles), N.ptr(None if vals is None else row_of),
+                                 N.ptr(vals), N.ptr(lkeys), N.ptr(col_ptr), N.ptr(row_idx), N.ptr(cvals), N.ptr(col_of), s),
+            "column_write")
+    return lkeys, col_ptr, row_idx, cvals, col_of
 
 
 def partition_by_key_range(keys: torch.Tensor, vals: Optional[torch.Tensor], separators) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:

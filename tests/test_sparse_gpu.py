@@ -113,3 +113,33 @@ def test_countmin_matches_host_and_set_ops_and_spmv():
     g = torch.empty(200_000, device="cuda")
     sparse.fill_gaussian(g, 1.0, 2.0, 7)
     assert abs(g.mean().item() - 1.0) < 0.03 and abs(g.std().item() - 2.0) < 0.03
+
+
+@pytest.mark.parametrize("valued", [False, True])
+@pytest.mark.parametrize("rows,per_row,keys", [(1, 1, 1), (3, 0, 5), (40, 51, 7), (64, 32, 1 << 40), (700, 90, 3000)])
+def test_columns_from_rows(rows, per_row, keys, valued):
+    from parameter_server_b200.ops import sparse
+
+    rng = np.random.RandomState(rows)
+    lens = rng.randint(0, 2 * per_row + 1, size=rows) if rows > 1 else np.array([per_row])
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    n = int(off[-1])
+    key = rng.randint(0, keys, size=n).astype(np.uint64) * np.uint64(0x9E3779B97F4A7C15)      # all eight bytes vary
+    val = rng.rand(n).astype(np.float32) if valued else None
+    d = lambda a: torch.from_numpy(a.view(np.int64) if a.dtype == np.uint64 else a).cuda()
+    lkeys, col_ptr, row_idx, vals, col_of = sparse.columns_from_rows(d(off), d(key), None if val is None else d(val))
+    order = np.argsort(key, kind="stable")
+    uk, cnt = np.unique(key, return_counts=True)
+    row_of = np.repeat(np.arange(rows), lens)
+    assert np.array_equal(lkeys.cpu().numpy().view(np.uint64), uk)
+    assert np.array_equal(col_ptr.cpu().numpy(), np.concatenate([[0], np.cumsum(cnt)]))
+    assert np.array_equal(row_idx.cpu().numpy(), row_of[order])
+    assert np.array_equal(col_of.cpu().numpy(), np.repeat(np.arange(len(uk)), cnt))
+    if valued:
+        assert np.array_equal(vals.cpu().numpy(), val[order])
+    else:
+        assert vals is None
+    # a shard of the rows: offsets that do not start at zero
+    assert torch.equal(sparse.columns_from_rows(d(off + 9), d(key), None)[2], row_idx)
+    with pytest.raises((ValueError, RuntimeError, IndexError)):      # rows that do not describe the non-zeros
+        sparse.columns_from_rows(d(np.concatenate([off[:-1], [n + 3]])), d(key), None)
