@@ -32,12 +32,9 @@ NVLINK_GBS = 770.0
 
 
 def main() -> None:
-    import ctypes as C
-
     import torch
 
     from parameter_server_b200.data.synthetic import mix64, zipf_ranks
-    from parameter_server_b200.ops import _native as N
     from parameter_server_b200.ops import sparse
     from parameter_server_b200.parallel.kv_vector import DeviceKVVector
     from parameter_server_b200.parallel.peer import PeerGroup
@@ -87,15 +84,7 @@ def main() -> None:
             t_pull = t_push = 0.0
             for it in range(args.warmup + iters):
                 if impl == "fused":
-                    M = eng._mb(mb)
-                    eng._L.parity = (eng.push_seq + 1) & 1
-                    ev[0].record()
-                    eng._launch_pull(M, insert=True)
-                    ev[1].record()
-                    eng.push_seq += 1
-                    N.check(eng._lib.psb_ftrl_push_update(C.byref(eng._P), C.byref(M), C.byref(eng._L), C.byref(eng._H),
-                                                          C.c_uint32(eng.push_seq), N.stream_ptr()), "ftrl_push_update")
-                    ev[2].record()
+                    eng.step(mb)     # one kernel; its own marks tell the pull from the rows and the push
                 else:
                     M = eng._mb(mb)
                     ev[0].record()
@@ -104,7 +93,11 @@ def main() -> None:
                     eng._push_nccl(M, *ctx)
                     ev[2].record()
                 torch.cuda.synchronize(dev)
-                if it >= args.warmup:
+                if it >= args.warmup and impl == "fused":
+                    ph = eng.phase_times_us()
+                    t_pull += (ph["localize"] + ph["lookup_reply"]) / 1e3
+                    t_push += (ph["rows"] + ph["flag_reset"] + ph["apply"]) / 1e3
+                elif it >= args.warmup:
                     t_pull += ev[0].elapsed_time(ev[1])
                     t_push += ev[1].elapsed_time(ev[2])
             eng.check_status()

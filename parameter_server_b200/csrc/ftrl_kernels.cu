@@ -1,24 +1,23 @@
-// Online FTRL-proximal on key-range sharded device hash tables: the two fused
+// Online FTRL-proximal on key-range sharded device hash tables: the fused
 // communication+compute kernels of the product path, plus the same phases as
 // stand-alone kernels for the unfused NCCL baseline.
 //
 // One rank = one GPU = worker r (streams minibatches) + server r (owns the keys
 // of [sep[r], sep[r+1]) in an open-addressing table {key -> w, z, pos, neg}).
+// A training step is one cooperative kernel, or two for a large minibatch:
 //
-//   ftrl_pull_spmv  : de-duplicate the minibatch's keys into a per-minibatch table
-//                     that is laid out by owner; every owner then reads "its" region
-//                     of every worker's table with coalesced peer loads over NVLink,
-//                     looks the keys up in its own shard (creating missing ones),
-//                     remembers the shard slot of every request and stores the
-//                     weights straight into the worker's weight array with coalesced
-//                     peer stores; the worker runs the CSR SpMV X·w, the logistic
-//                     loss and the per-row coefficient −y/(1+e^{y·Xw}) — one
-//                     cooperative kernel.
-//   ftrl_push_update: Xᵀ·coef and the pos/neg row counts per unique key into the
-//                     worker's accumulator array; every owner reads its region of
-//                     every worker's accumulators with coalesced peer loads and
-//                     applies the FTRL update to the slots it remembered, worker by
-//                     worker — one cooperative kernel.
+//   pull : de-duplicate the minibatch's keys into a per-minibatch table that is laid
+//          out by owner; every owner then reads "its" region of every worker's table
+//          with coalesced peer loads over NVLink, looks the keys up in its own shard
+//          (creating missing ones), remembers the shard slot of every request and
+//          stores the weights straight into the worker's weight array with coalesced
+//          peer stores.
+//   rows : row by row X·w, the logistic loss, the coefficient −y/(1+e^{y·Xw}) and at
+//          once the row's part of Xᵀ·coef and of the pos/neg row counts per unique
+//          key, into the worker's accumulator array.
+//   push : every owner reads its region of every worker's accumulators with coalesced
+//          peer loads and applies the FTRL update to the slots it remembered, worker
+//          by worker.
 //
 // No key is hashed twice on the owner, no record is packed, routed or copied into an
 // inbox: the per-minibatch table IS the message, and what crosses NVLink are whole
@@ -151,6 +150,21 @@ struct LocalScratch {
   // accesses of the gradient scatter then stay inside L2: a quarter of the footprint).
   uint32_t soa;
   uint32_t parity;     // which of the two accumulator buffers this step uses
+  uint32_t* region;    // state of the table's size, see below
+  int64_t two_launch_nnz;  // non-zeros from which on a step takes two launches (0: kTwoLaunchNnz)
+};
+
+// How much of the per-minibatch table a step uses.  The table is allocated for the largest minibatch the job may
+// send, but every slot of it is walked four times a step (owner lookup, owner update, key reset, accumulator
+// reset) and its keys and accumulators are probed at random, so a step works in the first 2^r slots only: r from
+// the minibatch's non-zeros (psb_ftrl_pull_spmv's `try_log2`), twice the slots as often as its keys do not fit.
+// One GPU only: with several, chunk c of every worker's table must cover the same key range.
+// B200, 10,000 rows (0.34 M keys) with the tail filter in 2^22 / 2^20 slots: step 264 / 167 us before the other changes;
+// 100,000 rows (2.4 M keys) in 2^24 / 2^22: 825 / 699 us.
+enum RegionWord : int {
+  kRegionNow = 0,       // log2 slots of the last pull; the push of the same step works in it too
+  kRegionFloor = 1,     // log2 slots that some minibatch of this engine needed: no step starts with fewer
+  kRegionMisfit = 2,    // log2 slots in which a pull's keys did not fit last
 };
 
 template <bool kCounts>
@@ -164,8 +178,8 @@ __device__ __forceinline__ size_t acc_bytes() { return kCounts ? sizeof(AccSlot)
 #define PSB_LD_F32(p, pol) ld_stream_f32((p), (pol))
 #define PSB_ST_U32(p, v, pol) st_stream_u32((p), (v), (pol))
 
-// trace slots: pull kernel 0 start, 1 localized, 2 all owners replied, 3 block-0 end;
-//              push kernel 4 start, 5 gradients done, 6 flags sent and tables cleared, 8 applied
+// trace slots: 0 start, 1 localized, 2 all owners replied, 3 rows done (a step: gradients too),
+//              4 flags sent and tables cleared, 5 applied
 #define PSB_TRACE(L, gtid, i) do { if ((L).trace != nullptr && (gtid) == 0) (L).trace[i] = globaltimer_ns(); } while (0)
 
 // Both tables index with the TOP bits of the same 64-bit hash (see FtrlPeers).
@@ -177,60 +191,116 @@ __device__ __forceinline__ uint64_t mb_key(const Minibatch& M, int64_t i, uint64
   return M.key_mode == 2 ? mix64(id) : id;
 }
 
-// slot of `key` in a per-minibatch table: region of its owner, top bits of its hash inside
-__device__ __forceinline__ uint64_t local_home(const FtrlPeers& P, uint64_t key) {
-  const uint64_t o = (uint64_t)route_owner(P.seps, key);
-  const uint64_t h = P.region_log2 ? (mix64(key) >> (64 - P.region_log2)) : 0ull;
-  return (o << P.region_log2) | h;
+// ------------------------------------------------------------------ phases
+// A non-zero's reference to its key: the slot, and the entry of the gradient cache that the key may use.  The entry
+// comes from the key's home in the WHOLE table, so which keys share an entry (and with it how their sums round) does
+// not depend on the slots that a step works in.  With more slots than kRefBits can tell, or several GPUs, the
+// reference is the slot alone and the entry is made from it.
+constexpr int kHotLog2 = 10;
+constexpr int kHotEntries = 1 << kHotLog2;
+constexpr uint32_t kRefBits = 32 - kHotLog2;
+__device__ __forceinline__ uint32_t hot_entry(uint32_t slot) { return (slot * 2654435761u) >> (32 - kHotLog2); }  // top bits
+struct Refs {
+  bool packed;
+  __device__ __forceinline__ Refs(const FtrlPeers& P, uint32_t rlog2) : packed(P.seps.world == 1 && rlog2 <= kRefBits) {}
+  __device__ __forceinline__ uint32_t make(uint32_t slot, uint32_t entry) const {
+    if (!packed || slot == kBadSlot) return slot;
+    const uint32_t ref = entry << kRefBits | slot;
+    return ref == kBadSlot ? ref - (1u << kRefBits) : ref;
+  }
+  __device__ __forceinline__ uint32_t slot(uint32_t ref) const { return packed ? ref & ((1u << kRefBits) - 1u) : ref; }
+  __device__ __forceinline__ uint32_t entry(uint32_t ref) const { return packed ? ref >> kRefBits : hot_entry(ref); }
+};
+
+// Home slot of `key` in a per-minibatch table (region of its owner, top bits of its hash inside) in the low half, its
+// cache entry in the high half.  A region has at least 4 slots.
+__device__ __forceinline__ uint64_t local_home(const FtrlPeers& P, uint64_t key, uint32_t rlog2) {
+  const uint64_t o = P.seps.world > 1 ? (uint64_t)route_owner(P.seps, key) : 0ull, x = mix64(key);
+  return (o << rlog2) | (x >> (64 - rlog2)) | (uint64_t)hot_entry((uint32_t)(x >> (64 - P.region_log2))) << 32;
 }
 
-// ------------------------------------------------------------------ phases
 // De-duplication of the minibatch's keys is bound by memory latency, not by bandwidth: every key
 // costs a streamed load of the key and then a dependent random read of the table.  The loop is
-// therefore software-pipelined: while key i is resolved, the table read of the thread's next key
-// and the load of the key after that are already in flight (the asm loads are issued in program
+// therefore software-pipelined: while a key is resolved, the table read of the thread's next key and the load of the
+// key after that are already in flight (the asm loads are issued in program
 // order, their results are used one and two iterations later).  A table read that is stale by the
 // time it is used only sends the key through the compare-and-swap path, which re-reads.
 __device__ __forceinline__ uint64_t ld_table_u64(const uint64_t* p) {
   uint64_t v; asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p)); return v;
 }
 
-__device__ __forceinline__ void phase_localize(const FtrlPeers& P, const Minibatch& M, const LocalScratch& L,
-                                               size_t gtid, size_t gsz) {
+// Slot of `key` in a per-minibatch table, entered when it is new; `cur` is what its home slot h held when it was read
+// (nothing is removed while keys are entered, so a stale value is an empty slot at worst, and the compare-and-swap
+// tells).  ~0 when the probe limit is hit.  (Looking at the home slot again cost an L2 request per new or displaced
+// key: 9.6 M non-zeros of 2.4 M keys in 2^23 slots 133 -> 110 us.)
+__device__ __forceinline__ uint64_t place_key(uint64_t* keys, uint64_t cmask, uint64_t h, uint64_t key, int max_probe, uint64_t cur,
+                                              uint32_t* fresh) {
+  const uint64_t base = h & ~cmask;
+  for (int i = 1;; ++i) {
+    if (cur == key) return h;
+    if (cur == kEmptyKey) {
+      cur = atomicCAS(reinterpret_cast<unsigned long long*>(keys + h), (unsigned long long)kEmptyKey, (unsigned long long)key);
+      if (cur == kEmptyKey) { ++*fresh; return h; }
+      if (cur == key) return h;
+    }
+    if (i >= max_probe) return ~0ull;
+    h = base | ((h + 1) & cmask);
+    cur = keys[h];
+  }
+}
+
+// Returns the number of keys this thread entered.  With fewer than 2^P.region_log2 slots a key that finds no
+// place leaves the size in the misfit word instead of an error, and the thread gives up: the caller starts over with
+// more slots.  kStreams: keys resolved at a time.
+template <int kStreams>
+__device__ __forceinline__ uint32_t phase_localize(const FtrlPeers& P, const Minibatch& M, const LocalScratch& L,
+                                                   size_t gtid, size_t gsz, uint32_t rlog2) {
   PSB_STREAM_POLICY(pol);
   const int64_t step = (int64_t)gsz;
-  const uint64_t region = 1ull << P.region_log2;
+  const uint64_t region = 1ull << rlog2;
   const uint64_t cmask = (region < (uint64_t)kChunkSlots ? region : (uint64_t)kChunkSlots) - 1;
+  const Refs refs(P, rlog2);
   uint32_t fresh = 0;
-  int64_t i = (int64_t)gtid;
-  if (i < M.nnz) {
-    uint64_t key0 = mb_key(M, i, pol);
-    uint64_t key1 = i + step < M.nnz ? mb_key(M, i + step, pol) : kEmptyKey;
-    uint64_t h0 = local_home(P, key0);
-    uint64_t cur0 = ld_table_u64(L.lt_keys + h0);
-    for (; i < M.nnz; i += step) {
-      uint64_t key2 = kEmptyKey, h1 = 0, cur1 = 0;
-      if (i + 2 * step < M.nnz) key2 = mb_key(M, i + 2 * step, pol);
-      if (i + step < M.nnz) {
-        h1 = local_home(P, key1);
-        cur1 = ld_table_u64(L.lt_keys + h1);
-      }
-      uint32_t slot = (uint32_t)h0;
-      if (cur0 != key0) {
-        bool inserted = false;
-        const uint64_t s = table_find_or_insert(L.lt_keys, ~0ull, cmask, h0, key0, P.max_probe, &inserted);
-        if (s == ~0ull) {
-          set_status(L.status, kLocalTableFull, 0, 0);
-          slot = kBadSlot;
-        } else {
-          slot = (uint32_t)s;
-          fresh += inserted ? 1u : 0u;
+  bool fits = true;
+  uint64_t key[kStreams], next[kStreams], h[kStreams], cur[kStreams];
+  const int64_t i0 = (int64_t)gtid;
+#pragma unroll
+  for (int j = 0; j < kStreams; ++j) {
+    const int64_t at = i0 + j * step, at1 = at + kStreams * step;
+    key[j] = at < M.nnz ? mb_key(M, at, pol) : kEmptyKey;
+    next[j] = at1 < M.nnz ? mb_key(M, at1, pol) : kEmptyKey;
+  }
+#pragma unroll
+  for (int j = 0; j < kStreams; ++j) {
+    h[j] = 0; cur[j] = 0;
+    if (i0 + j * step < M.nnz) { h[j] = local_home(P, key[j], rlog2); cur[j] = ld_table_u64(L.lt_keys + (uint32_t)h[j]); }
+  }
+  for (int64_t i = i0; i < M.nnz && fits; i += kStreams * step) {
+    uint64_t after[kStreams], nh[kStreams], ncur[kStreams];
+#pragma unroll
+    for (int j = 0; j < kStreams; ++j) {
+      const int64_t at1 = i + (kStreams + j) * step, at2 = at1 + kStreams * step;
+      after[j] = at2 < M.nnz ? mb_key(M, at2, pol) : kEmptyKey;
+      nh[j] = 0; ncur[j] = 0;
+      if (at1 < M.nnz) { nh[j] = local_home(P, next[j], rlog2); ncur[j] = ld_table_u64(L.lt_keys + (uint32_t)nh[j]); }
+    }
+#pragma unroll
+    for (int j = 0; j < kStreams; ++j) {
+      if (i + j * step < M.nnz) {
+        const uint64_t at = place_key(L.lt_keys, cmask, (uint32_t)h[j], key[j], P.max_probe, cur[j], &fresh);
+        if (at == ~0ull) {
+          if (rlog2 < P.region_log2) { L.region[kRegionMisfit] = rlog2; fits = false; }
+          else set_status(L.status, kLocalTableFull, 0, 0);
         }
+        PSB_ST_U32(L.slot_of + i + j * step, refs.make((uint32_t)at, (uint32_t)(h[j] >> 32)), pol);      // (uint32_t)~0 is kBadSlot
       }
-      PSB_ST_U32(L.slot_of + i, slot, pol);
-      key0 = key1; h0 = h1; cur0 = cur1; key1 = key2;
+      key[j] = next[j]; next[j] = after[j]; h[j] = nh[j]; cur[j] = ncur[j];
     }
   }
+  return fresh;
+}
+__device__ __forceinline__ void count_fresh(const LocalScratch& L, uint32_t fresh) {
+  __syncwarp();
   fresh = __reduce_add_sync(0xffffffffu, fresh);
   if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&L.stats[5], (double)fresh);
 }
@@ -290,10 +360,12 @@ constexpr int kLookupItems = kChunkSlots / 256;   // slots per thread and chunk 
 // Tasks are numbered sender-major starting with this rank itself, so the blocks that serve
 // different senders wait for different flags and a slow sender holds up only its own blocks.
 // `insert`: create missing keys (training); off for predictions and under the tail filter.
+// kAhead: home slots of the shard that are on their way before the first is looked at.
+template <int kAhead>
 __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScratch& L, uint32_t seq, bool insert,
-                                             int* sh_ok) {
+                                             uint32_t rlog2, int* sh_ok) {
   const int world = P.seps.world;
-  const uint64_t region = 1ull << P.region_log2;
+  const uint64_t region = 1ull << rlog2;
   const uint32_t chunk = region < (uint64_t)kChunkSlots ? (uint32_t)region : (uint32_t)kChunkSlots;
   const uint32_t chunks = (uint32_t)(region / chunk);
   const uint32_t tasks = chunks * (uint32_t)world;
@@ -308,8 +380,8 @@ __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScra
       have = s;
       if (!have_ok && threadIdx.x == 0) set_status(L.status, kWaitTimeout, (uint32_t)s, 1);
     }
-    const size_t in0 = ((size_t)s << P.region_log2) + (size_t)c * chunk;          // owner-side index
-    const size_t lt0 = ((size_t)P.rank << P.region_log2) + (size_t)c * chunk;     // index in the sender's table
+    const size_t in0 = ((size_t)s << rlog2) + (size_t)c * chunk;          // owner-side index
+    const size_t lt0 = ((size_t)P.rank << rlog2) + (size_t)c * chunk;     // index in the sender's table
     const bool peer = s != P.rank;
     const uint64_t* rk = P.lt_keys[s] + lt0;
     float* rw = P.lt_w[s] + lt0;
@@ -321,20 +393,37 @@ __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScra
       if (i < chunk && have_ok) key[k] = peer ? ld_relaxed_sys_u64(rk + i) : __ldcg(rk + i);
     }
 #pragma unroll
-    for (int k = 0; k < kLookupItems; ++k) {
-      const uint32_t i = (uint32_t)k * 256u + threadIdx.x;
-      if (i >= chunk) continue;
-      uint32_t slot = kBadSlot;
-      float w = 0.f;
-      if (key[k] != kEmptyKey) {
-        slot = insert ? shard_find_or_insert(P.tab, P.tab_mask, P.tab_shift, key[k], P.max_probe, &w, &dins)
-                      : shard_find(P.tab, P.tab_mask, P.tab_shift, key[k], P.max_probe, &w);
-        if (insert && slot == kAbsent) set_status(L.status, kShardTableFull, 0, 0);
+    for (int k = 0; k < kLookupItems; k += kAhead) {
+      uint64_t hk[kAhead], hw[kAhead];
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        hk[j] = kEmptyKey; hw[j] = 0ull;
+        if (kAhead > 1 && key[k + j] != kEmptyKey)
+          asm volatile("ld.global.v2.u64 {%0, %1}, [%2];" : "=l"(hk[j]), "=l"(hw[j])
+                       : "l"(P.tab + (shard_hash(key[k + j], P.tab_shift) & P.tab_mask)) : "memory");
       }
-      P.in_slot[in0 + i] = slot;
-      if (P.in_keys != nullptr) P.in_keys[in0 + i] = key[k];
-      if (have_ok) {
-        if (peer) st_relaxed_sys_f32(rw + i, w); else rw[i] = w;
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        const uint32_t i = (uint32_t)(k + j) * 256u + threadIdx.x;
+        if (i >= chunk) continue;
+        uint32_t slot = kBadSlot;
+        float w = 0.f;
+        if (key[k + j] != kEmptyKey) {
+          if (kAhead > 1 && hk[j] == key[k + j]) {
+            slot = (uint32_t)(shard_hash(key[k + j], P.tab_shift) & P.tab_mask);
+            w = __uint_as_float((uint32_t)hw[j]);
+          } else if (insert) {
+            slot = shard_find_or_insert(P.tab, P.tab_mask, P.tab_shift, key[k + j], P.max_probe, &w, &dins);
+            if (slot == kAbsent) set_status(L.status, kShardTableFull, 0, 0);
+          } else {
+            slot = kAhead > 1 && hk[j] == kEmptyKey ? kAbsent : shard_find(P.tab, P.tab_mask, P.tab_shift, key[k + j], P.max_probe, &w);
+          }
+        }
+        P.in_slot[in0 + i] = slot;
+        if (P.in_keys != nullptr) P.in_keys[in0 + i] = key[k + j];
+        if (have_ok) {
+          if (peer) st_relaxed_sys_f32(rw + i, w); else rw[i] = w;
+        }
       }
     }
   }
@@ -346,7 +435,7 @@ __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScra
 // non-zeros, then consumes them, so that several slot-map loads are in flight per lane.
 constexpr int kRowBatch = 4;
 
-__device__ __forceinline__ void phase_spmv_loss(const Minibatch& M, const LocalScratch& L, size_t gwarp,
+__device__ __forceinline__ void phase_spmv_loss(const Minibatch& M, const LocalScratch& L, const Refs refs, size_t gwarp,
                                                 size_t nwarps, int lane) {
   double loss = 0.0;
   PSB_STREAM_POLICY(pol);
@@ -364,7 +453,7 @@ __device__ __forceinline__ void phase_spmv_loss(const Minibatch& M, const LocalS
       }
 #pragma unroll
       for (int k = 0; k < kRowBatch; ++k) {
-        if (sl[k] != kBadSlot) s += x[k] * __ldcg(L.lt_w + sl[k]);   // written by other GPUs: not through L1
+        if (sl[k] != kBadSlot) s += x[k] * __ldcg(L.lt_w + refs.slot(sl[k]));   // written by other GPUs: not through L1
       }
     }
     s = warp_sum(s);
@@ -384,31 +473,67 @@ __device__ __forceinline__ void phase_spmv_loss(const Minibatch& M, const LocalS
 // shared memory and flushing once per block removes the same-address serialisation of
 // global atomics.  Entries are claimed first come, first served; a slot that finds its
 // cache line taken by another slot falls back to the global atomic.
-constexpr int kHotLog2 = 10;
-constexpr int kHotEntries = 1 << kHotLog2;
 struct HotCache {
   uint32_t slot[kHotEntries];
   float g[kHotEntries];
-  unsigned long long cnt[kHotEntries];
+  uint32_t pos[kHotEntries], neg[kHotEntries];   // native 32-bit shared-memory atomics; a block sees fewer than 2^31 non-zeros
 };
 
+// Adds gradients (and row counts) to the accumulators of this step through the block's cache.
 template <bool kCounts>
-__device__ __forceinline__ void phase_grad(const Minibatch& M, const LocalScratch& L, size_t gwarp,
-                                           size_t nwarps, int lane, HotCache* hc) {
-  float* accf = reinterpret_cast<float*>(L.lt_acc) + (size_t)L.parity * L.lt_slots;
-  AccSlot* accv = reinterpret_cast<AccSlot*>(L.lt_acc) + (size_t)L.parity * L.lt_slots;
-  for (int i = threadIdx.x; i < kHotEntries; i += blockDim.x) {
-    hc->slot[i] = kBadSlot;
-    hc->g[i] = 0.f;
-    if (kCounts) hc->cnt[i] = 0ull;
+struct HotScatter {
+  HotCache* hc;
+  float* accf;
+  AccSlot* accv;
+  __device__ __forceinline__ HotScatter(const LocalScratch& L, HotCache* h) : hc(h) {
+    accf = reinterpret_cast<float*>(L.lt_acc) + (size_t)L.parity * L.lt_slots;
+    accv = reinterpret_cast<AccSlot*>(L.lt_acc) + (size_t)L.parity * L.lt_slots;
+    for (int i = threadIdx.x; i < kHotEntries; i += blockDim.x) {
+      hc->slot[i] = kBadSlot;
+      hc->g[i] = 0.f;
+      if (kCounts) hc->pos[i] = hc->neg[i] = 0u;
+    }
+    __syncthreads();
   }
-  __syncthreads();
+  __device__ __forceinline__ void add(uint32_t sl, uint32_t h, float gv, bool is_pos) {
+    uint32_t cur = hc->slot[h];
+    if (cur == kBadSlot) {
+      const uint32_t prev = atomicCAS(&hc->slot[h], kBadSlot, sl);
+      cur = prev == kBadSlot ? sl : prev;
+    }
+    if (cur == sl) {
+      atomicAdd(&hc->g[h], gv);
+      if (kCounts) atomicAdd(is_pos ? &hc->pos[h] : &hc->neg[h], 1u);
+    } else if (kCounts) {
+      red_add_acc(accv + sl, gv, is_pos ? 1.f : 0.f, is_pos ? 0.f : 1.f);
+    } else {
+      atomicAdd(accf + sl, gv);
+    }
+  }
+  __device__ __forceinline__ void flush() {
+    __syncthreads();
+    for (int i = threadIdx.x; i < kHotEntries; i += blockDim.x) {
+      const uint32_t sl = hc->slot[i];
+      if (sl == kBadSlot) continue;
+      if (kCounts) {
+        red_add_acc(accv + sl, hc->g[i], (float)hc->pos[i], (float)hc->neg[i]);
+      } else {
+        atomicAdd(accf + sl, hc->g[i]);
+      }
+    }
+  }
+};
+
+// gradient alone, from stored coefficients (the unfused baseline)
+template <bool kCounts>
+__device__ __forceinline__ void phase_grad(const Minibatch& M, const LocalScratch& L, const Refs refs, size_t gwarp,
+                                           size_t nwarps, int lane, HotCache* hc) {
+  HotScatter<kCounts> scatter(L, hc);
   PSB_STREAM_POLICY(pol);
   for (int64_t row = (int64_t)gwarp; row < M.rows; row += (int64_t)nwarps) {
     const int64_t b = mb_offset(M, row), e = mb_offset(M, row + 1);
     const float c = L.coef[row];
     const bool is_pos = M.y[row] > 0.f;
-    const unsigned long long inc = is_pos ? (1ull << 32) : 1ull;
     for (int64_t i0 = b + lane; i0 < e; i0 += 32 * kRowBatch) {
       uint32_t sls[kRowBatch];
       float x[kRowBatch];
@@ -419,51 +544,79 @@ __device__ __forceinline__ void phase_grad(const Minibatch& M, const LocalScratc
         x[k] = (M.vals != nullptr && i < e) ? PSB_LD_F32(M.vals + i, pol) : 1.f;
       }
 #pragma unroll
+      for (int k = 0; k < kRowBatch; ++k)
+        if (sls[k] != kBadSlot) scatter.add(refs.slot(sls[k]), refs.entry(sls[k]), c * x[k], is_pos);
+    }
+  }
+  scatter.flush();
+}
+
+// A training step's rows, forward and backward in one walk: a warp multiplies a row with the pulled weights, has
+// the row's coefficient in registers and scatters the row's gradient at once.  The slots of a row's first
+// 32·kRowBatch non-zeros are read once and kept; the coefficient needs no array and the two halves no barrier.
+// B200, 100,000 rows: 239 us where X·w and gradient took 42 + 289 (16-byte accumulators, 2^22 slots against 2^24),
+// 187 us against 38 + 145 (4-byte).  Bound by the L2: a random weight sector and an atomic per non-zero.
+template <bool kCounts>
+__device__ __forceinline__ void phase_rows(const Minibatch& M, const LocalScratch& L, const Refs refs, size_t gwarp, size_t nwarps, int lane, HotCache* hc) {
+  HotScatter<kCounts> scatter(L, hc);
+  double loss = 0.0;
+  PSB_STREAM_POLICY(pol);
+  for (int64_t row = (int64_t)gwarp; row < M.rows; row += (int64_t)nwarps) {
+    const int64_t b = mb_offset(M, row), e = mb_offset(M, row + 1);
+    const float y = M.y[row];
+    uint32_t sl[kRowBatch];
+    float x[kRowBatch], s = 0.f;
+    for (int64_t i0 = b + lane, first = 1; first || i0 < e; i0 += 32 * kRowBatch, first = 0) {
+      uint32_t t[kRowBatch];
+      float v[kRowBatch];
+#pragma unroll
       for (int k = 0; k < kRowBatch; ++k) {
-        const uint32_t sl = sls[k];
-        if (sl == kBadSlot) continue;
-        const float gv = c * x[k];
-        const int h = (int)((sl * 2654435761u) >> (32 - kHotLog2));  // top bits
-        uint32_t cur = hc->slot[h];
-        if (cur == kBadSlot) {
-          const uint32_t prev = atomicCAS(&hc->slot[h], kBadSlot, sl);
-          cur = prev == kBadSlot ? sl : prev;
-        }
-        if (cur == sl) {
-          atomicAdd(&hc->g[h], gv);
-          if (kCounts) atomicAdd(&hc->cnt[h], inc);
-        } else if (kCounts) {
-          red_add_acc(accv + sl, gv, is_pos ? 1.f : 0.f, is_pos ? 0.f : 1.f);
-        } else {
-          atomicAdd(accf + sl, gv);
-        }
+        const int64_t i = i0 + 32 * k;
+        t[k] = i < e ? PSB_LD_U32(L.slot_of + i, pol) : kBadSlot;
+        v[k] = (M.vals != nullptr && i < e) ? PSB_LD_F32(M.vals + i, pol) : 1.f;
+      }
+#pragma unroll
+      for (int k = 0; k < kRowBatch; ++k) {
+        if (t[k] != kBadSlot) s += v[k] * __ldcg(L.lt_w + refs.slot(t[k]));   // written by other GPUs: not through L1
+        if (first) { sl[k] = t[k]; x[k] = v[k]; }
       }
     }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kHotEntries; i += blockDim.x) {
-    const uint32_t sl = hc->slot[i];
-    if (sl != kBadSlot) {
-      if (kCounts) {
-        const unsigned long long c = hc->cnt[i];
-        red_add_acc(accv + sl, hc->g[i], (float)(uint32_t)(c >> 32), (float)(uint32_t)c);
-      } else {
-        atomicAdd(accf + sl, hc->g[i]);
-      }
+    s = warp_sum(s);
+    const float m = y * s;
+    const float c = -y / (1.f + __expf(m));
+    if (lane == 0) {
+      loss += (double)log1pexp(-m);
+      L.xw[row] = s;
+    }
+    const bool is_pos = y > 0.f;
+#pragma unroll
+    for (int k = 0; k < kRowBatch; ++k)
+      if (sl[k] != kBadSlot) scatter.add(refs.slot(sl[k]), refs.entry(sl[k]), c * x[k], is_pos);
+    for (int64_t i = b + lane + 32 * kRowBatch; i < e; i += 32) {
+      const uint32_t t = PSB_LD_U32(L.slot_of + i, pol);
+      const float v = M.vals != nullptr ? PSB_LD_F32(M.vals + i, pol) : 1.f;
+      if (t != kBadSlot) scatter.add(refs.slot(t), refs.entry(t), c * v, is_pos);
     }
   }
+  if (lane == 0 && loss != 0.0) atomicAdd(&L.stats[0], loss);
+  scatter.flush();
 }
 
 // Between the gradient phase and the owners' update a worker empties its key table for the next
 // minibatch (every owner has finished reading it: the worker saw all `replied` flags before its
 // SpMV) and zeroes the accumulator buffer of the NEXT step (the owners read that one during the
 // previous step's update, which they finished before they replied to this step's pull).
-template <bool kCounts>
-__device__ __forceinline__ void phase_reset_tables(const LocalScratch& L, size_t gtid, size_t gsz) {
-  uint4* k = reinterpret_cast<uint4*>(L.lt_keys);
+__device__ __forceinline__ void clear_keys(uint64_t* keys, size_t slots, size_t gtid, size_t gsz) {
+  uint4* k = reinterpret_cast<uint4*>(keys);
   const uint4 empty = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-  for (size_t i = gtid; i < L.lt_slots / 2; i += gsz) k[i] = empty;
-  if (L.lt_slots & 1) { if (gtid == 0) L.lt_keys[L.lt_slots - 1] = kEmptyKey; }
+  for (size_t i = gtid; i < slots / 2; i += gsz) k[i] = empty;
+  if (slots & 1) { if (gtid == 0) keys[slots - 1] = kEmptyKey; }
+}
+// With one GPU nobody else reads the accumulators: the update zeroes each where it reads it and there is one buffer.
+template <bool kCounts>
+__device__ __forceinline__ void phase_reset_tables(const FtrlPeers& P, const LocalScratch& L, uint32_t rlog2, size_t gtid, size_t gsz) {
+  clear_keys(L.lt_keys, (size_t)P.seps.world << rlog2, gtid, gsz);
+  if (P.seps.world == 1) return;
   const size_t bytes = L.lt_slots * acc_bytes<kCounts>();
   char* next = reinterpret_cast<char*>(L.lt_acc) + (size_t)(L.parity ^ 1u) * bytes;
   uint4* a = reinterpret_cast<uint4*>(next);
@@ -525,15 +678,25 @@ __device__ __forceinline__ void apply_flush(ApplyAcc& a, double* stats) {
   a = ApplyAcc();
 }
 
-__device__ __forceinline__ void apply_slot(ShardSlot* tab, uint32_t slot, float g, uint32_t dpos, uint32_t dneg,
+// A slot is read and written as the 32-byte sector it is: one 256-bit access each way.  (Two 8-byte stores into a
+// sector cost the L2 twice the operations, and what a partial write evicts has to be merged in memory.)
+struct SlotWords { uint64_t key, wz, pn, reserved; };
+__device__ __forceinline__ SlotWords load_slot(const ShardSlot* p) {
+  SlotWords v;
+  asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.key), "=l"(v.wz), "=l"(v.pn), "=l"(v.reserved) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void store_slot(ShardSlot* p, const SlotWords& v) {
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v.key), "l"(v.wz), "l"(v.pn), "l"(v.reserved) : "memory");
+}
+// The key of a slot is written once, before any update of it, so storing it again changes nothing.
+__device__ __forceinline__ void apply_slot(ShardSlot* tab, uint32_t slot, SlotWords v, float g, uint32_t dpos, uint32_t dneg,
                                            const FtrlHyper& h, ApplyAcc& acc) {
-  const float2 wz = *reinterpret_cast<const float2*>(&tab[slot].w);
-  const uint2 pn = *reinterpret_cast<const uint2*>(&tab[slot].pos);
-  ShardState e;
-  e.w = wz.x; e.z = wz.y; e.pos = pn.x; e.neg = pn.y;
+  ShardState e{__uint_as_float((uint32_t)v.wz), __uint_as_float((uint32_t)(v.wz >> 32)), (uint32_t)v.pn, (uint32_t)(v.pn >> 32)};
   ftrl_update(e, g, dpos, dneg, h, acc.dn1, acc.dn2, acc.dnnz);
-  *reinterpret_cast<float2*>(&tab[slot].w) = make_float2(e.w, e.z);
-  *reinterpret_cast<uint2*>(&tab[slot].pos) = make_uint2(e.pos, e.neg);
+  v.wz = (uint64_t)__float_as_uint(e.z) << 32 | __float_as_uint(e.w);
+  v.pn = (uint64_t)e.neg << 32 | e.pos;
+  store_slot(tab + slot, v);
 }
 
 // gradient (and row counts) of request `i` of a chunk, from the sender's accumulators
@@ -554,14 +717,29 @@ __device__ __forceinline__ void load_acc(const void* base, size_t i, bool peer, 
   }
 }
 
+template <bool kCounts>
+__device__ __forceinline__ void zero_acc(void* base, size_t i) {
+  if (kCounts) reinterpret_cast<float4*>(base)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  else reinterpret_cast<float*>(base)[i] = 0.f;
+}
+
+// Lanes hold consecutive slots: does this lane's 32-byte sector of accumulators hold a used one?  Used sectors are
+// zeroed whole.  All 32 lanes call it.  (A partial write of a sector is much slower: 10 k rows in 2^22 slots, update
+// phase 433 us with the used 16 bytes alone, 169 us with all slots.)
+template <bool kCounts>
+__device__ __forceinline__ bool sector_used(bool used) {
+  const unsigned m = __ballot_sync(0xffffffffu, used);
+  return kCounts ? (m >> (threadIdx.x & 30) & 3u) != 0u : (m >> (threadIdx.x & 24) & 255u) != 0u;
+}
+
 // Owner side of the push: chunk c of every sender, sender by sender in rank order (the reference
 // applies each worker's push separately; the order only matters per key, and a key is in the
 // same chunk on every sender).  The shard slots were resolved by the pull of the same step.
 template <bool kCounts>
 __device__ __forceinline__ void phase_apply_chunks(const FtrlPeers& P, const LocalScratch& L, const FtrlHyper& H,
-                                                   uint32_t seq, ApplyAcc& acc, int* sh_ok) {
+                                                   uint32_t seq, uint32_t rlog2, ApplyAcc& acc, int* sh_ok) {
   const int world = P.seps.world;
-  const uint64_t region = 1ull << P.region_log2;
+  const uint64_t region = 1ull << rlog2;
   const uint32_t chunk = region < (uint64_t)kChunkSlots ? (uint32_t)region : (uint32_t)kChunkSlots;
   const uint32_t chunks = (uint32_t)(region / chunk);
   const size_t abytes = L.lt_slots * acc_bytes<kCounts>();
@@ -574,23 +752,34 @@ __device__ __forceinline__ void phase_apply_chunks(const FtrlPeers& P, const Loc
         if (!ok && threadIdx.x == 0) set_status(L.status, kWaitTimeout, (uint32_t)s, 2);
       }
       if (failed >> s & 1u) continue;   // a sender that never arrived is skipped
-      const size_t in0 = ((size_t)s << P.region_log2) + (size_t)c * chunk;
-      const size_t lt0 = ((size_t)P.rank << P.region_log2) + (size_t)c * chunk;
+      const size_t in0 = ((size_t)s << rlog2) + (size_t)c * chunk;
+      const size_t lt0 = ((size_t)P.rank << rlog2) + (size_t)c * chunk;
       const bool peer = s != P.rank;
-      const char* abase = reinterpret_cast<const char*>(P.lt_acc[s]) + (size_t)L.parity * abytes;
+      char* abase = reinterpret_cast<char*>(P.lt_acc[s]) + (size_t)L.parity * abytes;
       uint32_t slot[kLookupItems];
 #pragma unroll
       for (int k = 0; k < kLookupItems; ++k) {
         const uint32_t i = (uint32_t)k * 256u + threadIdx.x;
         slot[k] = i < chunk ? __ldcg(P.in_slot + in0 + i) : kBadSlot;
       }
+      // two slots at a time: the random reads of both sectors are in flight before the first is written (a sender's
+      // keys are distinct, so are their slots)
 #pragma unroll
-      for (int k = 0; k < kLookupItems; ++k) {
-        const uint32_t i = (uint32_t)k * 256u + threadIdx.x;
-        if (slot[k] >= kAbsent) continue;
-        float g; uint32_t dpos, dneg;
-        load_acc<kCounts>(abase, lt0 + i, peer, &g, &dpos, &dneg);
-        apply_slot(P.tab, slot[k], g, dpos, dneg, H, acc);
+      for (int k = 0; k < kLookupItems; k += 2) {
+        float g[2]; uint32_t dpos[2], dneg[2];
+        SlotWords e[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t i = (uint32_t)(k + j) * 256u + threadIdx.x;
+          if (slot[k + j] < kAbsent) {
+            e[j] = load_slot(P.tab + slot[k + j]);
+            load_acc<kCounts>(abase, lt0 + i, peer, &g[j], &dpos[j], &dneg[j]);
+          }
+          if (world == 1 && sector_used<kCounts>(slot[k + j] != kBadSlot) && i < chunk) zero_acc<kCounts>(abase, lt0 + i);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (slot[k + j] < kAbsent) apply_slot(P.tab, slot[k + j], e[j], g[j], dpos[j], dneg[j], H, acc);
       }
       __syncthreads();
     }
@@ -601,17 +790,18 @@ __device__ __forceinline__ void phase_apply_chunks(const FtrlPeers& P, const Loc
 // of its keys is queried, so every sender is bracketed by grid-wide barriers; keys that pass the
 // filter and have no entry yet get one here (the pull did not create them).
 __device__ __forceinline__ void phase_apply_filtered(cg::grid_group& grid, const FtrlPeers& P, const LocalScratch& L,
-                                                     const FtrlHyper& H, uint32_t seq, ApplyAcc& acc, int* sh_ok) {
+                                                     const FtrlHyper& H, uint32_t seq, uint32_t rlog2, ApplyAcc& acc,
+                                                     int* sh_ok) {
   const int world = P.seps.world;
-  const uint64_t region = 1ull << P.region_log2;
+  const uint64_t region = 1ull << rlog2;
   const size_t abytes = L.lt_slots * sizeof(AccSlot);
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, gsz = (size_t)gridDim.x * blockDim.x;
   for (int s = 0; s < world; ++s) {
     const bool ok = s == P.rank ? true : block_wait_flag(P.grads[P.rank] + s, seq, P.timeout_ns, sh_ok);
     if (!ok && threadIdx.x == 0) set_status(L.status, kWaitTimeout, (uint32_t)s, 2);
-    const size_t in0 = (size_t)s << P.region_log2, lt0 = (size_t)P.rank << P.region_log2;
+    const size_t in0 = (size_t)s << rlog2, lt0 = (size_t)P.rank << rlog2;
     const bool peer = s != P.rank;
-    const char* abase = reinterpret_cast<const char*>(P.lt_acc[s]) + (size_t)L.parity * abytes;
+    char* abase = reinterpret_cast<char*>(P.lt_acc[s]) + (size_t)L.parity * abytes;
     for (size_t i = gtid; ok && i < region; i += gsz) {
       const uint64_t key = P.in_keys[in0 + i];
       if (key == kEmptyKey) continue;
@@ -620,8 +810,14 @@ __device__ __forceinline__ void phase_apply_filtered(cg::grid_group& grid, const
       cm_insert(H.cm, H.cm_width, H.cm_k, key, dpos + dneg);
     }
     grid.sync();
-    for (size_t i = gtid; ok && i < region; i += gsz) {
-      const uint64_t key = P.in_keys[in0 + i];
+    const int lane = threadIdx.x & 31;
+    for (size_t i0 = gtid - lane; ok && i0 < region; i0 += gsz) {    // whole warps: a region may be shorter than one
+      const size_t i = i0 + lane;
+      const uint64_t key = i < region ? P.in_keys[in0 + i] : kEmptyKey;
+      float g = 0.f; uint32_t dpos = 0u, dneg = 0u;
+      if (key != kEmptyKey) load_acc<true>(abase, lt0 + i, peer, &g, &dpos, &dneg);
+      if (world == 1 && sector_used<true>(key != kEmptyKey) && i < region) zero_acc<true>(abase, lt0 + i);
+      __syncwarp();
       if (key == kEmptyKey) continue;
       if (cm_query(H.cm, H.cm_width, H.cm_k, key, 0xFFFFFFFFu) <= H.tail_freq) continue;
       uint32_t slot = __ldcg(P.in_slot + in0 + i);
@@ -630,41 +826,44 @@ __device__ __forceinline__ void phase_apply_filtered(cg::grid_group& grid, const
         slot = shard_find_or_insert(P.tab, P.tab_mask, P.tab_shift, key, P.max_probe, &w, &acc.dins);
         if (slot == kAbsent) { set_status(L.status, kShardTableFull, 0, 0); continue; }
       }
-      float g; uint32_t dpos, dneg;
-      load_acc<true>(abase, lt0 + i, peer, &g, &dpos, &dneg);
-      apply_slot(P.tab, slot, g, dpos, dneg, H, acc);
+      apply_slot(P.tab, slot, load_slot(P.tab + slot), g, dpos, dneg, H, acc);
     }
     grid.sync();
   }
 }
 
 // ------------------------------------------------------------ fused kernels
-// 8 blocks of 256 threads per SM (32 registers per thread): the phases of this kernel are bound by
-// memory latency and speed up with every resident warp.
-constexpr int kPullBlocksPerSM = 8;
 constexpr uint32_t kPullInsert = 1u;   // flags: create missing keys in the shard
+constexpr uint32_t kPullRows = 2u;     // ftrl_pull_kernel: multiply the rows too
 
-__global__ void __launch_bounds__(256, kPullBlocksPerSM)
-ftrl_pull_spmv_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_t flags) {
-  cg::grid_group grid = cg::this_grid();
-  const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t gsz = (size_t)gridDim.x * blockDim.x;
-  const int lane = threadIdx.x & 31;
+// De-duplication and lookup: the table is complete, every owner has been told, this rank's owner side has served
+// every worker, and every owner has served this one.  Returns the log2 slots worked in.
+template <int kStreams, int kAhead>
+__device__ __forceinline__ uint32_t pull_weights(cg::grid_group& grid, const FtrlPeers& P, const Minibatch& M, const LocalScratch& L,
+                                                 uint32_t seq, uint32_t flags, uint32_t try_log2, size_t gtid, size_t gsz, int* sh_ok) {
   const int world = P.seps.world;
-  __shared__ int sh_ok;
-
-  if (gtid == 0) L.stats[1] += (double)M.rows;
-  PSB_TRACE(L, gtid, 0);
-  phase_localize(P, M, L, gtid, gsz);
-  if (world > 1) __threadfence_system();   // the table must be visible to its owners before the flag is
-  grid.sync();
+  uint32_t rlog2 = world > 1 ? P.region_log2 : min(P.region_log2, max(try_log2, __ldcg(L.region + kRegionFloor)));
+  uint32_t fresh;
+  for (;;) {
+    fresh = phase_localize<kStreams>(P, M, L, gtid, gsz, rlog2);
+    if (world > 1) __threadfence_system();   // the table must be visible to its owners before the flag is
+    grid.sync();
+    // uniform: the word is written before the barrier above or, with another value, after the one below
+    if (rlog2 >= P.region_log2 || __ldcg(L.region + kRegionMisfit) != rlog2) break;
+    clear_keys(L.lt_keys, (size_t)1 << rlog2, gtid, gsz);
+    ++rlog2;
+    grid.sync();
+    if (gtid == 0) L.region[kRegionFloor] = rlog2;    // a size that did not fit is never tried again
+  }
+  count_fresh(L, fresh);
+  if (gtid == 0) L.region[kRegionNow] = rlog2;
   PSB_TRACE(L, gtid, 1);
   // this worker's table is complete: tell every owner, then serve the other workers' tables
   if (blockIdx.x == 0 && threadIdx.x < world && world > 1) {
     __threadfence_system();
     st_release_sys_u64(P.ready[threadIdx.x] + P.rank, (uint64_t)seq << 32);
   }
-  phase_lookup(P, L, seq, (flags & kPullInsert) != 0u, &sh_ok);
+  phase_lookup<kAhead>(P, L, seq, (flags & kPullInsert) != 0u, rlog2, sh_ok);
   if (world > 1) __threadfence_system();   // the weights must be visible to their workers before the flag is
   grid.sync();
   if (blockIdx.x == 0 && threadIdx.x < world && world > 1)
@@ -680,59 +879,83 @@ ftrl_pull_spmv_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, ui
     __syncthreads();
   }
   PSB_TRACE(L, gtid, 2);
-  phase_spmv_loss(M, L, gtid >> 5, gsz >> 5, lane);
-  PSB_TRACE(L, gtid, 3);
+  return rlog2;
 }
 
-// 6 blocks per SM (42 registers): measured best; 3 blocks (69 registers, no cap) and 8 blocks
-// (32 registers, spills) are both about 4 % slower per step.
-constexpr int kPushBlocksPerSM = 6;
-template <bool kCounts>
-__global__ void __launch_bounds__(256, kPushBlocksPerSM)
-ftrl_push_update_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t seq) {
+// The pull on its own: of a prediction (with X·w), and of a large training step.  8 blocks of 256 threads per SM (32
+// registers per thread): its phases are bound by memory latency and speed up with every resident warp.
+constexpr int kPullBlocksPerSM = 8;
+__global__ void __launch_bounds__(256, kPullBlocksPerSM)
+ftrl_pull_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_t flags, uint32_t try_log2) {
+  cg::grid_group grid = cg::this_grid();
+  const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t gsz = (size_t)gridDim.x * blockDim.x;
+  __shared__ int sh_ok;
+  if (gtid == 0) L.stats[1] += (double)M.rows;
+  PSB_TRACE(L, gtid, 0);
+  const uint32_t rlog2 = pull_weights<1, 1>(grid, P, M, L, seq, flags, try_log2, gtid, gsz, &sh_ok);
+  if (flags & kPullRows) {
+    phase_spmv_loss(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, threadIdx.x & 31);
+    PSB_TRACE(L, gtid, 3);
+  }
+}
+
+// A training step, whole (kPull) or after ftrl_pull_kernel: rows and push.
+constexpr int kStepBlocksPerSM = 5, kPushBlocksPerSM = 6;
+template <bool kCounts, bool kPull>
+__global__ void __launch_bounds__(256, kPull ? kStepBlocksPerSM : kPushBlocksPerSM)
+ftrl_step_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t pull_seq, uint32_t push_seq, uint32_t flags,
+                 uint32_t try_log2) {
   cg::grid_group grid = cg::this_grid();
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t gsz = (size_t)gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   const int world = P.seps.world;
-
   __shared__ HotCache hot;
   __shared__ int sh_ok;
-  PSB_TRACE(L, gtid, 4);
-  phase_grad<kCounts>(M, L, gtid >> 5, gsz >> 5, lane, &hot);
+
+  uint32_t rlog2;
+  if (kPull) {
+    if (gtid == 0) L.stats[1] += (double)M.rows;
+    PSB_TRACE(L, gtid, 0);
+    rlog2 = pull_weights<2, 2>(grid, P, M, L, pull_seq, flags, try_log2, gtid, gsz, &sh_ok);
+  } else {
+    rlog2 = __ldcg(L.region + kRegionNow);
+  }
+  phase_rows<kCounts>(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, lane, &hot);
   if (world > 1) __threadfence_system();   // the accumulators must be visible to their owners before the flag is
   grid.sync();
-  PSB_TRACE(L, gtid, 5);
+  PSB_TRACE(L, gtid, 3);
   if (blockIdx.x == 0 && threadIdx.x < world && world > 1)
-    st_release_sys_u64(P.grads[threadIdx.x] + P.rank, (uint64_t)seq << 32);
-  phase_reset_tables<kCounts>(L, gtid, gsz);
-  PSB_TRACE(L, gtid, 6);
+    st_release_sys_u64(P.grads[threadIdx.x] + P.rank, (uint64_t)push_seq << 32);
+  phase_reset_tables<kCounts>(P, L, rlog2, gtid, gsz);
+  PSB_TRACE(L, gtid, 4);
   {
     ApplyAcc acc;
     if (kCounts && tail_filter_on(H)) {
-      phase_apply_filtered(grid, P, L, H, seq, acc, &sh_ok);
+      phase_apply_filtered(grid, P, L, H, push_seq, rlog2, acc, &sh_ok);
     } else {
-      phase_apply_chunks<kCounts>(P, L, H, seq, acc, &sh_ok);
+      phase_apply_chunks<kCounts>(P, L, H, push_seq, rlog2, acc, &sh_ok);
     }
     apply_flush(acc, L.stats);
   }
-  PSB_TRACE(L, gtid, 8);
+  PSB_TRACE(L, gtid, 5);
 }
 
 // ------------------------------------------------- stand-alone phase kernels
 // (the unfused baseline: same arithmetic, records packed by owner and exchanged with all_to_all)
 __global__ void k_localize(FtrlPeers P, Minibatch M, LocalScratch L) {
-  phase_localize(P, M, L, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
+  count_fresh(L, phase_localize<1>(P, M, L, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, P.region_log2));
 }
-__global__ void k_spmv_loss(Minibatch M, LocalScratch L) {
+__global__ void k_spmv_loss(FtrlPeers P, Minibatch M, LocalScratch L) {
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gtid == 0) L.stats[1] += (double)M.rows;
-  phase_spmv_loss(M, L, gtid >> 5, ((size_t)gridDim.x * blockDim.x) >> 5, threadIdx.x & 31);
+  phase_spmv_loss(M, L, Refs(P, P.region_log2), gtid >> 5, ((size_t)gridDim.x * blockDim.x) >> 5, threadIdx.x & 31);
 }
-__global__ void k_grad(Minibatch M, LocalScratch L) {
+__global__ void k_grad(FtrlPeers P, Minibatch M, LocalScratch L) {
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   __shared__ HotCache hot;
-  phase_grad<true>(M, L, gtid >> 5, ((size_t)gridDim.x * blockDim.x) >> 5, threadIdx.x & 31, &hot);
+  phase_grad<true>(M, L, Refs(P, P.region_log2), gtid >> 5, ((size_t)gridDim.x * blockDim.x) >> 5, threadIdx.x & 31, &hot);
 }
 // count unique keys per owner (pass 1 of packing for all_to_all_v)
 __global__ void k_count_owner(KeySeps seps, LocalScratch L, uint32_t* counts) {
@@ -821,13 +1044,14 @@ __global__ void k_apply(ShardSlot* tab, uint64_t mask, uint32_t shift, int max_p
     const uint32_t slot = shard_find_or_insert(tab, mask, shift, key, max_probe, &w, &acc.dins);
     if (slot == kAbsent) { set_status(status, kShardTableFull, 0, 0); continue; }
     const uint64_t c = __ldcg(rc + i);
-    apply_slot(tab, slot, __ldcg(rg + i), (uint32_t)(c >> 32), (uint32_t)c, h, acc);
+    apply_slot(tab, slot, load_slot(tab + slot), __ldcg(rg + i), (uint32_t)(c >> 32), (uint32_t)c, h, acc);
   }
   apply_flush(acc, stats);
 }
-__global__ void k_clear_local(LocalScratch L) {
-  for (uint64_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x; s < L.lt_slots; s += (size_t)gridDim.x * blockDim.x)
-    L.lt_keys[s] = kEmptyKey;
+// empties the key table as far as the last pull used it
+__global__ void k_clear_local(LocalScratch L, int world) {
+  clear_keys(L.lt_keys, (size_t)world << L.region[kRegionNow], (size_t)blockIdx.x * blockDim.x + threadIdx.x,
+             (size_t)gridDim.x * blockDim.x);
 }
 // dump the non-zero weights of a shard: out_keys/out_w sized by capacity, *count receives the number
 __global__ void k_dump_nonzero(const ShardSlot* tab, uint64_t mask, uint64_t* out_keys,
@@ -863,7 +1087,7 @@ __global__ void k_rehash(const ShardSlot* from, uint64_t from_mask, ShardSlot* t
 using namespace psb;
 
 namespace {
-int g_coop_blocks_pull[16] = {0}, g_coop_blocks_push[2][16] = {{0}};
+int g_coop_blocks_pull[16] = {0}, g_coop_blocks_step[4][16] = {{0}};
 
 template <typename K>
 int coop_grid(K kernel, int* cache) {
@@ -889,43 +1113,85 @@ inline int flat_grid(size_t n, int cap = 148 * 8) {
 
 extern "C" {
 
-// flags bit 0: create missing keys in the shard (a training step; off for predictions)
-int psb_ftrl_pull_spmv(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, uint32_t seq, uint32_t flags,
-                       cudaStream_t stream) {
-  if (L->lt_w == nullptr || L->lt_acc == nullptr || P->in_slot == nullptr) return (int)cudaErrorInvalidValue;
-  const int grid = coop_grid(ftrl_pull_spmv_kernel, g_coop_blocks_pull);
-  if (grid <= 0) return (int)cudaErrorLaunchFailure;
-  FtrlPeers p = *P; Minibatch m = *M; LocalScratch l = *L;
-  void* args[] = {&p, &m, &l, &seq, &flags};
-  return (int)cudaLaunchCooperativeKernel((void*)ftrl_pull_spmv_kernel, dim3(grid), dim3(256), args, 0, stream);
+// log2 of the slots a minibatch starts with: three quarters of its non-zeros (a click stream has 0.25 to 0.5 distinct
+// keys per non-zero), but up to 2^17 slots, where walking the table costs next to nothing, four times the non-zeros.
+static uint32_t first_region_log2(int64_t nnz) {
+  const uint64_t n = nnz > 0 ? (uint64_t)nnz : 1ull;
+  const uint64_t small = n * 4 < 131072ull ? n * 4 : 131072ull;
+  const uint64_t want = n / 4 * 3 > small ? n / 4 * 3 : small;
+  uint32_t l = 2;
+  while ((1ull << l) < want) ++l;
+  // one more bit than a packed reference holds: three eighths will do
+  if (l == kRefBits + 1 && (1ull << kRefBits) >= n / 8 * 3) l = kRefBits;
+  return l;
 }
 
-int psb_ftrl_push_update(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, const FtrlHyper* H,
-                         uint32_t seq, cudaStream_t stream) {
+// Blocks of a launch: every grid-wide barrier costs more with more blocks, so a small minibatch gets one thread for
+// every two of its non-zeros and of the slots it works in (and at least a block per SM).
+static int step_grid(const FtrlPeers& P, const Minibatch& M, int full, uint32_t try_log2) {
+  if (P.seps.world > 1) return full;
+  const uint64_t slots = 1ull << (try_log2 < P.region_log2 ? try_log2 : P.region_log2);
+  const uint64_t n = (uint64_t)(M.nnz > 0 ? M.nnz : 0) > slots ? (uint64_t)M.nnz : slots;
+  const uint64_t want = (n + 511) / 512;
+  return want >= (uint64_t)full ? full : want < 148 ? (full < 148 ? full : 148) : (int)want;
+}
+
+static int launch_pull(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, uint32_t seq, uint32_t flags, cudaStream_t stream) {
+  uint32_t try_log2 = first_region_log2(M->nnz);
+  const int full = coop_grid(ftrl_pull_kernel, g_coop_blocks_pull);
+  if (full <= 0) return (int)cudaErrorLaunchFailure;
+  const int grid = step_grid(*P, *M, full, try_log2);
+  FtrlPeers p = *P; Minibatch m = *M; LocalScratch l = *L;
+  void* args[] = {&p, &m, &l, &seq, &flags, &try_log2};
+  return (int)cudaLaunchCooperativeKernel((void*)ftrl_pull_kernel, dim3(grid), dim3(256), args, 0, stream);
+}
+
+// A prediction: X·w with the weights as they are, no key is created.
+int psb_ftrl_pull_spmv(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, uint32_t seq, cudaStream_t stream) {
+  if (L->lt_w == nullptr || L->lt_acc == nullptr || P->in_slot == nullptr || L->region == nullptr) return (int)cudaErrorInvalidValue;
+  return launch_pull(P, M, L, seq, kPullRows, stream);
+}
+
+// Non-zeros from which on a step takes two launches.
+constexpr int64_t kTwoLaunchNnz = 3000000;
+
+// One training step: pull, rows, push (sequence numbers of the pull's and the push's flags).  flags bit 0: create
+// missing keys in the shard.
+int psb_ftrl_step(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, const FtrlHyper* H, uint32_t pull_seq,
+                  uint32_t push_seq, uint32_t flags, cudaStream_t stream) {
   const bool soa = L->soa != 0;
   const bool filter = H->tail_freq != 0u && H->cm != nullptr;
+  if (L->lt_w == nullptr || L->lt_acc == nullptr || P->in_slot == nullptr || L->region == nullptr) return (int)cudaErrorInvalidValue;
   // the count-based rule and the tail filter need the pos/neg counts that the one-float accumulators do not carry
   if (soa && (H->rule == 0 || filter)) return (int)cudaErrorInvalidValue;
   if (filter && P->in_keys == nullptr) return (int)cudaErrorInvalidValue;
-  void* kernel = soa ? (void*)ftrl_push_update_kernel<false> : (void*)ftrl_push_update_kernel<true>;
-  const int grid = soa ? coop_grid(ftrl_push_update_kernel<false>, g_coop_blocks_push[0])
-                       : coop_grid(ftrl_push_update_kernel<true>, g_coop_blocks_push[1]);
-  if (grid <= 0) return (int)cudaErrorLaunchFailure;
+  const bool two = M->nnz >= (L->two_launch_nnz > 0 ? L->two_launch_nnz : kTwoLaunchNnz);
+  if (two) {
+    const int e = launch_pull(P, M, L, pull_seq, flags & kPullInsert, stream);
+    if (e != 0) return e;
+  }
+  const void* kernels[4] = {(const void*)ftrl_step_kernel<false, false>, (const void*)ftrl_step_kernel<true, false>,
+                            (const void*)ftrl_step_kernel<false, true>, (const void*)ftrl_step_kernel<true, true>};
+  const int which = (soa ? 0 : 1) + (two ? 0 : 2);
+  const int full = coop_grid(kernels[which], g_coop_blocks_step[which]);
+  if (full <= 0) return (int)cudaErrorLaunchFailure;
+  uint32_t try_log2 = first_region_log2(M->nnz);
+  const int grid = step_grid(*P, *M, full, try_log2);
   FtrlPeers p = *P; Minibatch m = *M; LocalScratch l = *L; FtrlHyper h = *H;
-  void* args[] = {&p, &m, &l, &h, &seq};
-  return (int)cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(256), args, 0, stream);
+  void* args[] = {&p, &m, &l, &h, &pull_seq, &push_seq, &flags, &try_log2};
+  return (int)cudaLaunchCooperativeKernel(kernels[which], dim3(grid), dim3(256), args, 0, stream);
 }
 
 int psb_ftrl_localize(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, cudaStream_t s) {
   k_localize<<<flat_grid(M->nnz), 256, 0, s>>>(*P, *M, *L);
   return (int)cudaGetLastError();
 }
-int psb_ftrl_spmv_loss(const Minibatch* M, const LocalScratch* L, cudaStream_t s) {
-  k_spmv_loss<<<flat_grid((size_t)M->rows * 32), 256, 0, s>>>(*M, *L);
+int psb_ftrl_spmv_loss(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, cudaStream_t s) {
+  k_spmv_loss<<<flat_grid((size_t)M->rows * 32), 256, 0, s>>>(*P, *M, *L);
   return (int)cudaGetLastError();
 }
-int psb_ftrl_grad(const Minibatch* M, const LocalScratch* L, cudaStream_t s) {
-  k_grad<<<flat_grid((size_t)M->rows * 32), 256, 0, s>>>(*M, *L);
+int psb_ftrl_grad(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, cudaStream_t s) {
+  k_grad<<<flat_grid((size_t)M->rows * 32), 256, 0, s>>>(*P, *M, *L);
   return (int)cudaGetLastError();
 }
 int psb_ftrl_count_owner(const KeySeps* seps, const LocalScratch* L, uint32_t* counts, cudaStream_t s) {
@@ -958,8 +1224,8 @@ int psb_ftrl_apply(void* tab, uint64_t mask, uint32_t shift, int max_probe, cons
   k_apply<<<flat_grid(n), 256, 0, s>>>((ShardSlot*)tab, mask, shift, max_probe, rk, rg, rc, n, *h, stats, status);
   return (int)cudaGetLastError();
 }
-int psb_ftrl_clear_local(const LocalScratch* L, cudaStream_t s) {
-  k_clear_local<<<flat_grid(L->lt_slots), 256, 0, s>>>(*L);
+int psb_ftrl_clear_local(const LocalScratch* L, int world, cudaStream_t s) {
+  k_clear_local<<<flat_grid(L->lt_slots), 256, 0, s>>>(*L, world);
   return (int)cudaGetLastError();
 }
 int psb_ftrl_dump_nonzero(const void* tab, uint64_t mask, uint64_t* out_keys, float* out_w,

@@ -3,13 +3,14 @@
 Role map to the reference: :class:`FTRLEngine` is worker + server of one rank —
 ``FTRL::updateModel`` (src/linear_method/ftrl.cc:61-152) on the worker side and
 ``FTRLModel`` (src/linear_method/ftrl_model.h) on the server side.  A step is
-two cooperative kernels (see ``csrc/ftrl_kernels.cu``):
+one cooperative kernel (see ``csrc/ftrl_kernels.cu``), which pulls, multiplies and pushes:
 
-* pull-fused SpMV  — dedup keys into a table laid out by owner; every owner reads its region
+* pull  — dedup keys into a table laid out by owner; every owner reads its region
   of every worker's table over NVLink, looks the keys up in its shard and stores the weights
-  into the worker's weight array; ``Xw``, logistic loss, per-row coefficient;
-* push-fused update — ``Xᵀ·coef`` + pos/neg counts per unique key into the worker's
-  accumulators; every owner reads its region of them over NVLink and applies the FTRL update
+  into the worker's weight array;
+* rows  — ``Xw``, logistic loss, per-row coefficient and at once ``Xᵀ·coef`` + pos/neg counts
+  per unique key into the worker's accumulators;
+* push  — every owner reads its region of them over NVLink and applies the FTRL update
   to the shard slots it resolved during the pull.
 
 ``impl="nccl"`` runs the same arithmetic with stand-alone kernels and
@@ -127,7 +128,9 @@ class FTRLEngine:
         # --- worker side, readable / writable by the owners: per-minibatch table, weights, accumulators, flags
         self.lt_keys = group.alloc((self.lcap,), i64, fill=-1)
         self.lt_w = group.alloc((self.lcap,), f32)
-        self.lt_acc = group.alloc((2, self.lcap, 4) if self.track_counts else (2, self.lcap), f32)
+        # several GPUs: two buffers in turn, since the owners read one while the other is zeroed
+        buffers = 2 if W > 1 else 1
+        self.lt_acc = group.alloc((buffers, self.lcap, 4) if self.track_counts else (buffers, self.lcap), f32)
         self.ready = group.alloc((N.MAX_RANKS,), i64)
         self.replied = group.alloc((N.MAX_RANKS,), i64)
         self.grads = group.alloc((N.MAX_RANKS,), i64)
@@ -176,6 +179,11 @@ class FTRLEngine:
         L.send_cnt, L.recv_cnt = self.send_cnt.data_ptr(), self.recv_cnt.data_ptr()
         L.stats, L.status = self.stats.data_ptr(), self.status.data_ptr()
         L.trace = self.trace.data_ptr()
+        # [0] log2 slots of the table that the last pull used, [1] log2 slots known to be needed, [2] log2 slots that did
+        # not fit (csrc/ftrl_kernels.cu, RegionWord)
+        self.region = torch.zeros((8,), dtype=torch.int32, device=d)
+        self.region[0] = self.region_log2
+        L.region = self.region.data_ptr()
         L.soa = 0 if self.track_counts else 1
         self._L = L
         self._H = hyper.native()
@@ -267,24 +275,19 @@ class FTRLEngine:
             raise RuntimeError(f"rank {self.group.rank}: {N.STATUS_NAMES.get(st[0], st[0])} (peer/arg={st[1]}, phase={st[2]})")
 
     # -------------------------------------------------------------------- step
-    def _launch_pull(self, M, insert: bool) -> None:
-        self.pull_seq += 1
-        N.check(self._lib.psb_ftrl_pull_spmv(C.byref(self._P), C.byref(M), C.byref(self._L), C.c_uint32(self.pull_seq),
-                                             C.c_uint32(1 if insert else 0), N.stream_ptr()), "ftrl_pull_spmv")
-        self.kernel_launches += 1
-
     def step(self, mb: DeviceMinibatch) -> None:
         """Enqueue one training step on the current stream (no host synchronisation)."""
         if self.impl == "nccl":
             return self._step_nccl(mb)
         self.epoch += 1
         M = self._mb(mb)
-        self._L.parity = (self.push_seq + 1) & 1
-        # under the tail filter a key gets its entry only when it passes the filter, in the push
-        self._launch_pull(M, insert=self.hyper.tail_feature_freq <= 0)
+        self.pull_seq += 1
         self.push_seq += 1
-        N.check(self._lib.psb_ftrl_push_update(C.byref(self._P), C.byref(M), C.byref(self._L), C.byref(self._H),
-                                               C.c_uint32(self.push_seq), N.stream_ptr()), "ftrl_push_update")
+        self._L.parity = self.push_seq & 1 if self.group.world > 1 else 0
+        # under the tail filter a key gets its entry only when it passes the filter, in the push
+        insert = 1 if self.hyper.tail_feature_freq <= 0 else 0
+        N.check(self._lib.psb_ftrl_step(C.byref(self._P), C.byref(M), C.byref(self._L), C.byref(self._H), C.c_uint32(self.pull_seq),
+                                        C.c_uint32(self.push_seq), C.c_uint32(insert), N.stream_ptr()), "ftrl_step")
         self.kernel_launches += 1
 
     def predict(self, mb: DeviceMinibatch) -> torch.Tensor:
@@ -296,8 +299,11 @@ class FTRLEngine:
             self.group.barrier()   # every owner's last apply kernel has finished
             self._pull_nccl(M)
         else:
-            self._launch_pull(M, insert=False)
-        N.check(self._lib.psb_ftrl_clear_local(C.byref(self._L), s), "clear_local")
+            self.pull_seq += 1
+            N.check(self._lib.psb_ftrl_pull_spmv(C.byref(self._P), C.byref(M), C.byref(self._L), C.c_uint32(self.pull_seq),
+                                                 s), "ftrl_pull_spmv")
+            self.kernel_launches += 1
+        N.check(self._lib.psb_ftrl_clear_local(C.byref(self._L), self.group.world, s), "clear_local")
         self.kernel_launches += 1
         out = self.xw[: mb.rows].clone()
         self.stats.copy_(saved)
@@ -351,7 +357,7 @@ class FTRLEngine:
             uw = rw
         if total:
             N.check(lib.psb_ftrl_scatter_w(N.ptr(self._u_slot), N.ptr(uw), C.c_uint32(total), C.byref(L), s), "scatter_w")
-        N.check(lib.psb_ftrl_spmv_loss(C.byref(M), C.byref(L), s), "spmv_loss")
+        N.check(lib.psb_ftrl_spmv_loss(C.byref(self._P), C.byref(M), C.byref(L), s), "spmv_loss")
         self.kernel_launches += 2
         return counts, in_counts, rkeys
 
@@ -361,7 +367,7 @@ class FTRLEngine:
 
         lib, L, s = self._lib, self._L, N.stream_ptr()
         W, total, nr = self.group.world, sum(counts), rkeys.numel()
-        N.check(lib.psb_ftrl_grad(C.byref(M), C.byref(L), s), "grad")
+        N.check(lib.psb_ftrl_grad(C.byref(self._P), C.byref(M), C.byref(L), s), "grad")
         ug = torch.empty((total,), dtype=torch.float32, device=self.dev)
         uc = torch.empty((total,), dtype=torch.int64, device=self.dev)
         if total:
@@ -397,11 +403,12 @@ class FTRLEngine:
                 "unique_keys": v[5], "table_entries": v[6]}
 
     def phase_times_us(self) -> dict:
-        """Durations (µs) of the phases of the last fused step, from in-kernel globaltimer marks."""
+        """Durations (µs) of the phases of the last fused step, from in-kernel globaltimer marks; "rows" is X·w, the
+        loss and the gradients."""
         t = self.trace.tolist()
         d = lambda a, b: (t[b] - t[a]) / 1e3
-        return {"localize": d(0, 1), "lookup_reply": d(1, 2), "spmv_loss": d(2, 3), "kernel_gap": d(3, 4), "grad": d(4, 5),
-                "flag_reset": d(5, 6), "apply": d(6, 8), "step": d(0, 8)}
+        return {"localize": d(0, 1), "lookup_reply": d(1, 2), "rows": d(2, 3), "flag_reset": d(3, 4), "apply": d(4, 5),
+                "step": d(0, 5)}
 
     def penalty(self, st: dict) -> float:
         """λ₁‖w‖₁ + ½λ₂·sqrt(‖w‖₂²) exactly as FTRLModel::objv (src/linear_method/ftrl_model.h:31)."""

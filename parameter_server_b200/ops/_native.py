@@ -59,7 +59,8 @@ class LocalScratch(C.Structure):
     _fields_ = [("lt_keys", C.c_void_p), ("lt_w", C.c_void_p), ("lt_acc", C.c_void_p), ("lt_slots", C.c_uint64),
                 ("slot_of", C.c_void_p), ("coef", C.c_void_p), ("xw", C.c_void_p),
                 ("send_cnt", C.c_void_p), ("recv_cnt", C.c_void_p), ("stats", C.c_void_p),
-                ("status", C.c_void_p), ("trace", C.c_void_p), ("soa", C.c_uint32), ("parity", C.c_uint32)]
+                ("status", C.c_void_p), ("trace", C.c_void_p), ("soa", C.c_uint32), ("parity", C.c_uint32),
+                ("region", C.c_void_p), ("two_launch_nnz", C.c_int64)]
 
 
 def lib() -> C.CDLL:

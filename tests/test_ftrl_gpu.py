@@ -115,6 +115,66 @@ def test_ftrl_reports_local_table_overflow():
         eng.check_status()
 
 
+@pytest.mark.parametrize("rule", ["count", "sumsq"])
+def test_minibatches_of_changing_size_and_one_without_repeated_keys(rule):
+    """A step works in as many slots as its minibatch suggests and starts over with more when the keys do not fit;
+    the accumulators of a large step are clean when a later step goes as far again."""
+    from parameter_server_b200.models.ftrl import DeviceMinibatch
+
+    eng, hy = _engine(rule=rule, table_capacity=1 << 21, local_capacity=1 << 20, max_rows=8192)
+    ref = FTRLRef(hy.alpha, hy.beta, hy.lambda1, hy.lambda2, rule)
+    small, large = _batches(1, rows=60)[0], _batches(1, rows=2000)[0]
+    # all keys distinct: 2^18 slots, which three quarters of the non-zeros ask for, cannot hold 300,000
+    g = torch.Generator(device="cuda").manual_seed(5)
+    keys = torch.randperm(1 << 22, generator=g, device="cuda")[:300_000] * 0x9E3779B9
+    off = torch.arange(0, 300_001, 60, device="cuda")
+    y = torch.where(torch.rand(5000, generator=g, device="cuda") < 0.5, 1.0, -1.0)
+    distinct = (off, keys, y)
+    used = []
+    for off, keys, y in [large, small, large, small, distinct, small, small, distinct, large]:
+        eng.step(DeviceMinibatch(off, keys, y))
+        eng.check_status()
+        used.append(int(eng.region[0].item()))
+        ref.step([(off.cpu().numpy(), keys.cpu().numpy().view(np.uint64), y.cpu().numpy().astype(np.float64))])
+        xw = eng.predict(DeviceMinibatch(*small)).cpu().numpy()
+        rxw = ref.worker_gradient(small[0].cpu().numpy(), small[1].cpu().numpy().view(np.uint64), small[2].cpu().numpy().astype(np.float64))[5]
+        np.testing.assert_allclose(xw, rxw, rtol=2e-3, atol=2e-4)
+    assert used[1] < used[0] < used[4] <= eng.region_log2 and used[5] == used[4], used
+    k, w = eng.dump_model()
+    rk, rw = ref.nonzero()
+    assert np.array_equal(k, rk)
+    np.testing.assert_allclose(w, rw, rtol=2e-3, atol=2e-5)
+    assert int((eng.lt_keys.local != -1).sum()) == 0
+    assert eng.read_stats(reset=False)["table_entries"] == len(ref.model)
+
+
+@pytest.mark.parametrize("valued", [False, True])
+@pytest.mark.parametrize("rule", ["count", "sumsq"])
+def test_rows_of_all_lengths(rule, valued):
+    """Rows without non-zeros, around one warp and around what a warp keeps in registers, and far longer ones."""
+    from parameter_server_b200.models.ftrl import DeviceMinibatch
+
+    eng, hy = _engine(rule=rule)
+    ref = FTRLRef(hy.alpha, hy.beta, hy.lambda1, hy.lambda2, rule)
+    rng = np.random.RandomState(4)
+    for lens in ([0], [1], [0, 1, 31, 32, 33, 0, 127, 128, 129, 160, 1000, 0], [5] * 3000, [129] * 17):
+        off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+        keys = rng.randint(0, 900, size=off[-1]).astype(np.int64) * 0x9E3779B97F
+        y = np.where(rng.rand(len(lens)) < 0.4, 1.0, -1.0).astype(np.float32)
+        vals = (rng.rand(off[-1]) + 0.5).astype(np.float32) if valued else None
+        d = lambda a: None if a is None else torch.from_numpy(a).cuda()
+        eng.step(DeviceMinibatch(d(off), d(keys), d(y), d(vals)))
+        eng.check_status()
+        want = ref.worker_gradient(off, keys.view(np.uint64), y.astype(np.float64), vals)[5] if off[-1] else np.zeros(len(lens))
+        np.testing.assert_allclose(eng.xw[: len(lens)].cpu().numpy(), want, rtol=2e-3, atol=2e-4)
+        if off[-1]:
+            ref.step([(off, keys.view(np.uint64), y.astype(np.float64)) + ((vals,) if valued else ())])
+    k, w = eng.dump_model()
+    rk, rw = ref.nonzero()
+    assert np.array_equal(k, rk)
+    np.testing.assert_allclose(w, rw, rtol=2e-3, atol=2e-5)
+
+
 def test_model_text_dump(tmp_path):
     from parameter_server_b200.models.ftrl import DeviceMinibatch
     from parameter_server_b200.utils.modelio import read_model_text
