@@ -251,8 +251,7 @@ __device__ __forceinline__ uint64_t place_key(uint64_t* keys, uint64_t cmask, ui
 
 // Returns the number of keys this thread entered.  With fewer than 2^P.region_log2 slots a key that finds no
 // place leaves the size in the misfit word instead of an error, and the thread gives up: the caller starts over with
-// more slots.  kStreams: keys resolved at a time.
-template <int kStreams>
+// more slots.
 __device__ __forceinline__ uint32_t phase_localize(const FtrlPeers& P, const Minibatch& M, const LocalScratch& L,
                                                    size_t gtid, size_t gsz, uint32_t rlog2) {
   PSB_STREAM_POLICY(pol);
@@ -261,48 +260,54 @@ __device__ __forceinline__ uint32_t phase_localize(const FtrlPeers& P, const Min
   const uint64_t cmask = (region < (uint64_t)kChunkSlots ? region : (uint64_t)kChunkSlots) - 1;
   const Refs refs(P, rlog2);
   uint32_t fresh = 0;
-  bool fits = true;
-  uint64_t key[kStreams], next[kStreams], h[kStreams], cur[kStreams];
-  const int64_t i0 = (int64_t)gtid;
-#pragma unroll
-  for (int j = 0; j < kStreams; ++j) {
-    const int64_t at = i0 + j * step, at1 = at + kStreams * step;
-    key[j] = at < M.nnz ? mb_key(M, at, pol) : kEmptyKey;
-    next[j] = at1 < M.nnz ? mb_key(M, at1, pol) : kEmptyKey;
-  }
-#pragma unroll
-  for (int j = 0; j < kStreams; ++j) {
-    h[j] = 0; cur[j] = 0;
-    if (i0 + j * step < M.nnz) { h[j] = local_home(P, key[j], rlog2); cur[j] = ld_table_u64(L.lt_keys + (uint32_t)h[j]); }
-  }
-  for (int64_t i = i0; i < M.nnz && fits; i += kStreams * step) {
-    uint64_t after[kStreams], nh[kStreams], ncur[kStreams];
-#pragma unroll
-    for (int j = 0; j < kStreams; ++j) {
-      const int64_t at1 = i + (kStreams + j) * step, at2 = at1 + kStreams * step;
-      after[j] = at2 < M.nnz ? mb_key(M, at2, pol) : kEmptyKey;
-      nh[j] = 0; ncur[j] = 0;
-      if (at1 < M.nnz) { nh[j] = local_home(P, next[j], rlog2); ncur[j] = ld_table_u64(L.lt_keys + (uint32_t)nh[j]); }
+  int64_t i = (int64_t)gtid;
+  if (i >= M.nnz) return 0u;
+  uint64_t key0 = mb_key(M, i, pol);
+  uint64_t key1 = i + step < M.nnz ? mb_key(M, i + step, pol) : kEmptyKey;
+  uint64_t h0 = local_home(P, key0, rlog2);
+  uint64_t cur0 = ld_table_u64(L.lt_keys + (uint32_t)h0);
+  for (; i < M.nnz; i += step) {
+    uint64_t key2 = kEmptyKey, h1 = 0, cur1 = 0;
+    if (i + 2 * step < M.nnz) key2 = mb_key(M, i + 2 * step, pol);
+    if (i + step < M.nnz) {
+      h1 = local_home(P, key1, rlog2);
+      cur1 = ld_table_u64(L.lt_keys + (uint32_t)h1);
     }
-#pragma unroll
-    for (int j = 0; j < kStreams; ++j) {
-      if (i + j * step < M.nnz) {
-        const uint64_t at = place_key(L.lt_keys, cmask, (uint32_t)h[j], key[j], P.max_probe, cur[j], &fresh);
-        if (at == ~0ull) {
-          if (rlog2 < P.region_log2) { L.region[kRegionMisfit] = rlog2; fits = false; }
-          else set_status(L.status, kLocalTableFull, 0, 0);
-        }
-        PSB_ST_U32(L.slot_of + i + j * step, refs.make((uint32_t)at, (uint32_t)(h[j] >> 32)), pol);      // (uint32_t)~0 is kBadSlot
-      }
-      key[j] = next[j]; next[j] = after[j]; h[j] = nh[j]; cur[j] = ncur[j];
+    const uint64_t at = place_key(L.lt_keys, cmask, (uint32_t)h0, key0, P.max_probe, cur0, &fresh);
+    if (at == ~0ull) {
+      if (rlog2 < P.region_log2) { L.region[kRegionMisfit] = rlog2; break; }
+      set_status(L.status, kLocalTableFull, 0, 0);
     }
+    PSB_ST_U32(L.slot_of + i, refs.make((uint32_t)at, (uint32_t)(h0 >> 32)), pol);      // (uint32_t)~0 is kBadSlot
+    key0 = key1; h0 = h1; cur0 = cur1; key1 = key2;
   }
   return fresh;
 }
-__device__ __forceinline__ void count_fresh(const LocalScratch& L, uint32_t fresh) {
-  __syncwarp();
-  fresh = __reduce_add_sync(0xffffffffu, fresh);
-  if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(&L.stats[5], (double)fresh);
+// Adds a block's values to stats[at], ..., stats[at + kN - 1] with one fp64 atomic each; every thread of the block calls
+// it.  (One per warp, thousands of warps wait in line at one address: 20 us of a 600 us step at each use.)
+template <int kN>
+__device__ __forceinline__ void block_add(double* stats, const int (&at)[kN], const double (&v)[kN]) {
+  __shared__ double sh[8][kN];     // blocks of 256 threads
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kN; ++k) {
+    const double s = warp_sum_d(v[k]);
+    if (lane == 0) sh[warp][k] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kN; ++k) {
+    if (threadIdx.x != k) continue;
+    double s = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += sh[w][k];
+    if (s != 0.0) atomicAdd(stats + at[k], s);
+  }
+}
+__device__ __forceinline__ void block_add1(double* stats, int at, double v) {
+  const int a[1] = {at};
+  const double x[1] = {v};
+  block_add<1>(stats, a, x);
 }
 
 // ---- shard table probes (owner side, this GPU's own memory)
@@ -427,8 +432,7 @@ __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScra
       }
     }
   }
-  dins = __reduce_add_sync(0xffffffffu, dins);
-  if ((threadIdx.x & 31) == 0 && dins) atomicAdd(&L.stats[6], (double)dins);
+  if (insert) block_add1(L.stats, 6, (double)dins);
 }
 
 // Rows are walked a warp at a time; a lane first issues the loads of up to kRowBatch of its
@@ -465,7 +469,7 @@ __device__ __forceinline__ void phase_spmv_loss(const Minibatch& M, const LocalS
       L.xw[row] = s;
     }
   }
-  if (lane == 0 && loss != 0.0) atomicAdd(&L.stats[0], loss);
+  block_add1(L.stats, 0, loss);      // (lane 0 has the row's loss, the others zero)
 }
 
 // Block-local cache of gradient accumulators for frequently hit slots.  Under Zipf
@@ -598,7 +602,7 @@ __device__ __forceinline__ void phase_rows(const Minibatch& M, const LocalScratc
       if (t != kBadSlot) scatter.add(refs.slot(t), refs.entry(t), c * v, is_pos);
     }
   }
-  if (lane == 0 && loss != 0.0) atomicAdd(&L.stats[0], loss);
+  block_add1(L.stats, 0, loss);      // (lane 0 has the row's loss, the others zero)
   scatter.flush();
 }
 
@@ -667,14 +671,9 @@ struct ApplyAcc {  // per-thread deltas of the model statistics, flushed once pe
 };
 
 __device__ __forceinline__ void apply_flush(ApplyAcc& a, double* stats) {
-  const float dn1 = warp_sum(a.dn1), dn2 = warp_sum(a.dn2);
-  const int dnnz = __reduce_add_sync(0xffffffffu, a.dnnz), dins = __reduce_add_sync(0xffffffffu, a.dins);
-  if ((threadIdx.x & 31) == 0) {
-    if (dn1 != 0.f) atomicAdd(stats + 2, (double)dn1);
-    if (dn2 != 0.f) atomicAdd(stats + 3, (double)dn2);
-    if (dnnz != 0) atomicAdd(stats + 4, (double)dnnz);
-    if (dins != 0) atomicAdd(stats + 6, (double)dins);
-  }
+  const int at[4] = {2, 3, 4, 6};
+  const double v[4] = {(double)a.dn1, (double)a.dn2, (double)a.dnnz, (double)a.dins};
+  block_add<4>(stats, at, v);
   a = ApplyAcc();
 }
 
@@ -838,14 +837,14 @@ constexpr uint32_t kPullRows = 2u;     // ftrl_pull_kernel: multiply the rows to
 
 // De-duplication and lookup: the table is complete, every owner has been told, this rank's owner side has served
 // every worker, and every owner has served this one.  Returns the log2 slots worked in.
-template <int kStreams, int kAhead>
+template <int kAhead>
 __device__ __forceinline__ uint32_t pull_weights(cg::grid_group& grid, const FtrlPeers& P, const Minibatch& M, const LocalScratch& L,
                                                  uint32_t seq, uint32_t flags, uint32_t try_log2, size_t gtid, size_t gsz, int* sh_ok) {
   const int world = P.seps.world;
   uint32_t rlog2 = world > 1 ? P.region_log2 : min(P.region_log2, max(try_log2, __ldcg(L.region + kRegionFloor)));
   uint32_t fresh;
   for (;;) {
-    fresh = phase_localize<kStreams>(P, M, L, gtid, gsz, rlog2);
+    fresh = phase_localize(P, M, L, gtid, gsz, rlog2);
     if (world > 1) __threadfence_system();   // the table must be visible to its owners before the flag is
     grid.sync();
     // uniform: the word is written before the barrier above or, with another value, after the one below
@@ -855,7 +854,7 @@ __device__ __forceinline__ uint32_t pull_weights(cg::grid_group& grid, const Ftr
     grid.sync();
     if (gtid == 0) L.region[kRegionFloor] = rlog2;    // a size that did not fit is never tried again
   }
-  count_fresh(L, fresh);
+  block_add1(L.stats, 5, (double)fresh);
   if (gtid == 0) L.region[kRegionNow] = rlog2;
   PSB_TRACE(L, gtid, 1);
   // this worker's table is complete: tell every owner, then serve the other workers' tables
@@ -893,7 +892,7 @@ ftrl_pull_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_
   __shared__ int sh_ok;
   if (gtid == 0) L.stats[1] += (double)M.rows;
   PSB_TRACE(L, gtid, 0);
-  const uint32_t rlog2 = pull_weights<1, 1>(grid, P, M, L, seq, flags, try_log2, gtid, gsz, &sh_ok);
+  const uint32_t rlog2 = pull_weights<1>(grid, P, M, L, seq, flags, try_log2, gtid, gsz, &sh_ok);
   if (flags & kPullRows) {
     phase_spmv_loss(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, threadIdx.x & 31);
     PSB_TRACE(L, gtid, 3);
@@ -918,7 +917,7 @@ ftrl_step_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t
   if (kPull) {
     if (gtid == 0) L.stats[1] += (double)M.rows;
     PSB_TRACE(L, gtid, 0);
-    rlog2 = pull_weights<2, 2>(grid, P, M, L, pull_seq, flags, try_log2, gtid, gsz, &sh_ok);
+    rlog2 = pull_weights<2>(grid, P, M, L, pull_seq, flags, try_log2, gtid, gsz, &sh_ok);
   } else {
     rlog2 = __ldcg(L.region + kRegionNow);
   }
@@ -945,7 +944,8 @@ ftrl_step_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t
 // ------------------------------------------------- stand-alone phase kernels
 // (the unfused baseline: same arithmetic, records packed by owner and exchanged with all_to_all)
 __global__ void k_localize(FtrlPeers P, Minibatch M, LocalScratch L) {
-  count_fresh(L, phase_localize<1>(P, M, L, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, P.region_log2));
+  const uint32_t fresh = phase_localize(P, M, L, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, P.region_log2);
+  block_add1(L.stats, 5, (double)fresh);
 }
 __global__ void k_spmv_loss(FtrlPeers P, Minibatch M, LocalScratch L) {
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1152,8 +1152,10 @@ int psb_ftrl_pull_spmv(const FtrlPeers* P, const Minibatch* M, const LocalScratc
   return launch_pull(P, M, L, seq, kPullRows, stream);
 }
 
-// Non-zeros from which on a step takes two launches.
-constexpr int64_t kTwoLaunchNnz = 3000000;
+// Non-zeros from which on a step takes two launches: the pull gains more from its own 8 blocks per SM than the second
+// launch costs.  B200, step in one / two launches (count rule): 48 k non-zeros 44 / 48 us, 1 M 185 / 190, 2.9 M 325 / 315,
+// 5.3 M 432 / 419, 9.6 M 738 / 670.
+constexpr int64_t kTwoLaunchNnz = 1500000;
 
 // One training step: pull, rows, push (sequence numbers of the pull's and the push's flags).  flags bit 0: create
 // missing keys in the shard.
