@@ -1,12 +1,12 @@
 // Dense layer GEMM on the 5th-generation tensor cores: D[M,N] = act(A[M,K] · B[N,K]ᵀ), fp32 in
 // memory, TF32 multiply, fp32 accumulate in tensor memory (TMEM).
 //
-// One CTA (128 threads) per 128x128 output tile:
+// Small and medium problems: one CTA (128 threads) per 128x128 output tile:
 //   warp 0, one lane   TMA producer: cp.async.bulk.tensor 2-D tiles of A and B (128 rows x 32 floats =
-//                      one 128-byte swizzle row each) into a 4-stage shared-memory ring, completion on
-//                      the stage's "full" mbarrier
-//   warp 1, one lane   MMA issuer: tcgen05.mma.cta_group::1.kind::tf32, four K=8 steps per stage, the
-//                      accumulator lives in 128 TMEM columns; tcgen05.commit releases the stage
+//                      one 128-byte swizzle row each, two spans per stage) into a 3-stage shared-memory
+//                      ring, completion on the stage's "full" mbarrier
+//   warp 1, one lane   MMA issuer: tcgen05.mma.cta_group::1.kind::tf32, eight K=8 steps per stage (with
+//                      four, the barriers' round trips were a third of the time), the accumulator lives in 128 TMEM columns; tcgen05.commit releases the stage
 //                      ("empty" mbarrier) and finally signals "accumulator complete"
 //   all 4 warps        epilogue: tcgen05.ld 32 lanes x 32 columns per warp and step, activation, store
 // Both operands are K-major (row-major with K contiguous), which is how the layers keep their data:
@@ -26,9 +26,8 @@
 namespace psb {
 
 constexpr int kBM = 128, kBN = 128, kBK = 32;       // tile; kBK floats = 128 bytes = swizzle span
-constexpr int kStages = 4;
+constexpr int kStages = 3, kSpans = 2;
 constexpr int kUmmaK = 8;                            // K per tcgen05.mma for tf32
-constexpr uint32_t kStageBytesA = kBM * kBK * 4, kStageBytesB = kBN * kBK * 4;
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kWaitLimit = 4u * 1000u * 1000u;   // polls of try_wait before giving up
 
@@ -89,22 +88,66 @@ __device__ __forceinline__ float apply_act(float x, int act) {
   }
 }
 
+// 32 columns of one row (lane = row, registers = columns) through the activation to out and, when out_t is given,
+// to its transpose [N, M]: for a fixed column the lanes of a warp hold consecutive rows, so those stores are
+// whole 128-byte lines and cost no second pass over the matrix.
+__device__ __forceinline__ void store_chunk(const uint32_t (&r)[32], float* __restrict__ out, float* __restrict__ out_t, int row, int col,
+                                            int M, int N, int ldo, int act) {
+  if (row >= M || col >= N) return;
+  float* dst = out + (size_t)row * ldo + col;
+  float* dst_t = out_t != nullptr ? out_t + (size_t)col * M + row : nullptr;
+  const int ncol = N - col;
+  if (ncol >= 32 && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+      float4 v;
+      v.x = apply_act(__uint_as_float(r[j]), act);
+      v.y = apply_act(__uint_as_float(r[j + 1]), act);
+      v.z = apply_act(__uint_as_float(r[j + 2]), act);
+      v.w = apply_act(__uint_as_float(r[j + 3]), act);
+      *reinterpret_cast<float4*>(dst + j) = v;
+      if (dst_t != nullptr) {
+        dst_t[(size_t)j * M] = v.x;
+        dst_t[(size_t)(j + 1) * M] = v.y;
+        dst_t[(size_t)(j + 2) * M] = v.z;
+        dst_t[(size_t)(j + 3) * M] = v.w;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < ncol) {
+        const float v = apply_act(__uint_as_float(r[j]), act);
+        dst[j] = v;
+        if (dst_t != nullptr) dst_t[(size_t)j * M] = v;
+      }
+  }
+}
+
 struct __align__(1024) GemmSmem {
-  float a[kStages][kBM * kBK];
-  float b[kStages][kBN * kBK];
+  float a[kStages][kSpans][kBM * kBK];
+  float b[kStages][kSpans][kBN * kBK];
   uint64_t full[kStages], empty[kStages], acc_full;
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
 };
 
+// kRows: rows of A that exist and are loaded (the tile's other rows are whatever shared memory holds: rows do not
+// mix, and theirs are not stored); kCols: columns of the tile.  The weight gradient of a layer with one output is
+// [1, batch] · [batch, in]: a few CTAs walk all of K one block after the other.  With 8 rows and 32 columns a block
+// is an eighth of the loads and there are four times the CTAs; the sums and their order stay the same.
+// B200, L2 flushed, before and after (one 32-deep block per barrier, square tiles): 1x1024x8192 106 -> 64 us,
+// 1024x1024x8192 107 -> 80, 4096x1024x8192 211 -> 154.
+constexpr int kThinRows = 8, kThinCols = 32;
+template <int kRows, int kCols>
 __global__ void __launch_bounds__(128, 1)
 gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                         float* __restrict__ out, int M, int N, int K, int ldo, int act, uint32_t* status) {
+                         float* __restrict__ out, float* __restrict__ out_t, int M, int N, int K, int ldo, int act, uint32_t* status) {
   extern __shared__ uint8_t smem_raw[];
   GemmSmem& s = *reinterpret_cast<GemmSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
-  const int nkb = (K + kBK - 1) / kBK;
+  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kCols;
+  const int nkb = (K + kSpans * kBK - 1) / (kSpans * kBK);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], 1); }
@@ -126,29 +169,33 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     for (int kb = 0; kb < nkb; ++kb) {
       const int st = kb % kStages;
       if (kb >= kStages && !mbar_wait(&s.empty[st], ((kb / kStages) - 1) & 1)) { s.abort_flag = 1; break; }
-      if (s.abort_flag) break;
-      mbar_expect_tx(&s.full[st], kStageBytesA + kStageBytesB);
-      tma_load_2d(s.a[st], &map_a, &s.full[st], kb * kBK, m0);
-      tma_load_2d(s.b[st], &map_b, &s.full[st], kb * kBK, n0);
+      mbar_expect_tx(&s.full[st], (uint32_t)(kRows + kCols) * kSpans * kBK * 4);
+#pragma unroll
+      for (int h = 0; h < kSpans; ++h) {       // a span past the end of K is filled with zeros
+        tma_load_2d(s.a[st][h], &map_a, &s.full[st], (kb * kSpans + h) * kBK, m0);
+        tma_load_2d(s.b[st][h], &map_b, &s.full[st], (kb * kSpans + h) * kBK, n0);
+      }
     }
   } else if (warp == 1 && lane == 0) {
     // ---------------- MMA issuer
-    constexpr uint32_t idesc = make_idesc(kBM, kBN);
+    constexpr uint32_t idesc = make_idesc(kBM, kCols);
     for (int kb = 0; kb < nkb; ++kb) {
       const int st = kb % kStages;
       if (!mbar_wait(&s.full[st], (kb / kStages) & 1)) { s.abort_flag = 1; break; }
-      if (s.abort_flag) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint64_t da = make_smem_desc(smem_u32(s.a[st]));
-      const uint64_t db = make_smem_desc(smem_u32(s.b[st]));
 #pragma unroll
-      for (int k = 0; k < kBK / kUmmaK; ++k) {
-        const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
-        const uint64_t adv = (uint64_t)((k * kUmmaK * 4) >> 4);   // 32 bytes per K step inside the swizzle row
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem), "l"(da + adv), "l"(db + adv), "r"(idesc), "r"(accumulate) : "memory");
+      for (int h = 0; h < kSpans; ++h) {
+        const uint64_t da = make_smem_desc(smem_u32(s.a[st][h]));
+        const uint64_t db = make_smem_desc(smem_u32(s.b[st][h]));
+#pragma unroll
+        for (int k = 0; k < kBK / kUmmaK; ++k) {
+          const uint32_t accumulate = (kb > 0 || h > 0 || k > 0) ? 1u : 0u;
+          const uint64_t adv = (uint64_t)((k * kUmmaK * 4) >> 4);   // 32 bytes per K step inside the swizzle row
+          asm volatile(
+              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+              "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+              ::"r"(tmem), "l"(da + adv), "l"(db + adv), "r"(idesc), "r"(accumulate) : "memory");
+        }
       }
       // release the stage once the MMAs that read it have completed
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s.empty[st])) : "memory");
@@ -169,7 +216,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (ok) {
     const int row = m0 + warp * 32 + lane;
 #pragma unroll 1
-    for (int c0 = 0; c0 < kBN; c0 += 32) {
+    for (int c0 = 0; c0 < kCols; c0 += 32) {
       uint32_t r[32];
       const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
       asm volatile(
@@ -182,25 +229,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
           : "r"(taddr) : "memory");
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (row < M) {
-        float* dst = out + (size_t)row * ldo + n0 + c0;
-        const int ncol = N - (n0 + c0);
-        if (ncol >= 32 && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            float4 v;
-            v.x = apply_act(__uint_as_float(r[j]), act);
-            v.y = apply_act(__uint_as_float(r[j + 1]), act);
-            v.z = apply_act(__uint_as_float(r[j + 2]), act);
-            v.w = apply_act(__uint_as_float(r[j + 3]), act);
-            *reinterpret_cast<float4*>(dst + j) = v;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < ncol) dst[j] = apply_act(__uint_as_float(r[j]), act);
-        }
-      }
+      store_chunk(r, out, out_t, row, n0 + c0, M, N, ldo, act);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -216,80 +245,107 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   }
 }
 
-// ------------------------------------------------------------------ persistent variant for large problems
-// One CTA per SM walks a list of 128x256 output tiles.  Six warps: warp 0 (one lane) TMA producer,
-// warp 1 (one lane) MMA issuer, warps 2-5 epilogue (warp w reads TMEM lanes 32·(w mod 4) ...).  The
-// accumulator is double-buffered in TMEM (2 x 256 columns): while the epilogue warps drain tile i, the
-// tensor core already works on tile i+1.  The shared-memory ring runs across tile boundaries.
-constexpr int kPBN = 256;
-constexpr int kPStages = 4;
-constexpr uint32_t kPStageBytesB = kPBN * kBK * 4;
-constexpr int kPThreads = 192;
+// ------------------------------------------------------------------ CTA pairs
+// Large problems: persistent pairs of SMs, each pair on one 256x256 tile at a time (cta_group::2): a CTA holds 128
+// rows of A and 128 of the 256 rows of B, and the tensor cores of both read B from both shared memories, so an SM
+// loads 32 KB per 32-deep K block instead of the 48 KB that a 128x256 tile of its own takes, and six stages fit.
+// The accumulator is double-buffered in TMEM (2 x 256 columns): the epilogue of a tile runs under the next tile's
+// main loop.  What bounds it is how fast one thread gets K blocks through its barriers (a read of the abort flag per K
+// block cost a seventh of the rate at K = 8192) and, for short K, writing the result.  TF32 rates on B200, L2 flushed
+// between calls, against 128x256 tiles on single persistent CTAs: 4096x1024x8192 524 -> 645 TFLOP/s, 8192x4096x1024
+// 513 -> 550, 3000x3000x2044 370 -> 472.
+//   both CTAs   warp 0: TMA loads of the CTA's own halves, completion counted on the LEADER's "full" barrier
+//   leader      warp 1: tcgen05.mma for the pair; its commits release the stage ("empty") and publish the
+//               accumulator ("tfull") in both CTAs
+//   both CTAs   warps 2-5: epilogue of the CTA's 128 rows; they hand the accumulator back on the leader's "tempty"
+// Every CTA loads its own rows: no multicast load.
+constexpr int kDTile = 256, kDHalf = 128, kDStages = 6, kPThreads = 192;
+constexpr uint32_t kDHalfBytes = kDHalf * kBK * 4;
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-struct __align__(1024) GemmSmemP {
-  float a[kPStages][kBM * kBK];
-  float b[kPStages][kPBN * kBK];
-  uint64_t full[kPStages], empty[kPStages], tfull[2], tempty[2];
+struct __align__(1024) GemmSmemD {
+  float a[kDStages][kDHalf * kBK];
+  float b[kDStages][kDHalf * kBK];
+  uint64_t full[kDStages], empty[kDStages], tfull[2], tempty[2];
   uint32_t tmem_base;
   volatile uint32_t abort_flag;
 };
 
-__global__ void __launch_bounds__(kPThreads, 1)
-gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                            float* __restrict__ out, int M, int N, int K, int ldo, int act, uint32_t* status) {
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
+  uint32_t r; asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank)); return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// bar: shared::cluster address of a barrier in either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+// arrive on the barrier at this offset in both CTAs once the MMAs issued so far have completed
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
+gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                      float* __restrict__ out, float* __restrict__ out_t, int M, int N, int K, int ldo, int act, uint32_t* status) {
   extern __shared__ uint8_t smem_raw[];
-  GemmSmemP& s = *reinterpret_cast<GemmSmemP*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  GemmSmemD& s = *reinterpret_cast<GemmSmemD*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nbm = (M + kBM - 1) / kBM, nbn = (N + kPBN - 1) / kPBN;
-  const int ntiles = nbm * nbn;
+  const int rank = (int)cluster_rank();
+  const int nbm = (M + kDTile - 1) / kDTile, nbn = (N + kDTile - 1) / kDTile;
+  const int ntiles = nbm * nbn, pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int nkb = (K + kBK - 1) / kBK;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kPStages; ++i) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&s.tfull[i], 1); mbar_init(&s.tempty[i], 4); }
+    for (int i = 0; i < kDStages; ++i) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s.tfull[i], 1); mbar_init(&s.tempty[i], 8); }
     s.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem_base)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  cluster_sync_all();       // the peer's barriers are ready before anything is signalled there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = s.tmem_base;
 
   if (warp == 0 && lane == 0) {
-    // ---------------- TMA producer: tiles are walked m-fastest so that concurrent CTAs share a B panel
+    // ---------------- TMA producer, tiles m-fastest
     uint32_t g = 0;
-    for (int t = blockIdx.x; t < ntiles && !s.abort_flag; t += gridDim.x) {
-      const int m0 = (t % nbm) * kBM, n0 = (t / nbm) * kPBN;
+    for (int t = pair; t < ntiles && !s.abort_flag; t += npairs) {
+      const int m0 = (t % nbm) * kDTile + rank * kDHalf, n0 = (t / nbm) * kDTile + rank * kDHalf;
       for (int kb = 0; kb < nkb; ++kb, ++g) {
-        const int st = g % kPStages;
-        if (g >= (uint32_t)kPStages && !mbar_wait(&s.empty[st], ((g / kPStages) - 1) & 1)) { s.abort_flag = 1; break; }
-        if (s.abort_flag) break;
-        mbar_expect_tx(&s.full[st], kStageBytesA + kPStageBytesB);
-        tma_load_2d(s.a[st], &map_a, &s.full[st], kb * kBK, m0);
-        tma_load_2d(s.b[st], &map_b, &s.full[st], kb * kBK, n0);
+        const int st = g % kDStages;
+        if (g >= (uint32_t)kDStages && !mbar_wait(&s.empty[st], ((g / kDStages) - 1) & 1)) { s.abort_flag = 1; break; }
+        if (rank == 0) mbar_expect_tx(&s.full[st], 4 * kDHalfBytes);
+        const uint32_t bar = mapa_u32(smem_u32(&s.full[st]), 0);
+        tma_load_2d_pair(s.a[st], &map_a, bar, kb * kBK, m0);
+        tma_load_2d_pair(s.b[st], &map_b, bar, kb * kBK, n0);
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ---------------- MMA issuer
-    constexpr uint32_t idesc = make_idesc(kBM, kPBN);
+    // the last releases must have landed here before this CTA's shared memory may go away
+    for (uint32_t u = g > (uint32_t)kDStages ? g - kDStages : 0; u < g && !s.abort_flag; ++u)
+      if (!mbar_wait(&s.empty[u % kDStages], (u / kDStages) & 1)) s.abort_flag = 1;
+  } else if (warp == 1 && lane == 0 && rank == 0) {
+    // ---------------- MMA issuer of the pair
+    constexpr uint32_t idesc = make_idesc(kDTile, kDTile);
     uint32_t g = 0, it = 0;
-    for (int t = blockIdx.x; t < ntiles && !s.abort_flag; t += gridDim.x, ++it) {
+    for (int t = pair; t < ntiles && !s.abort_flag; t += npairs, ++it) {
       const uint32_t acc = it & 1u;
       if (it >= 2 && !mbar_wait(&s.tempty[acc], ((it >> 1) - 1) & 1)) { s.abort_flag = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t d_tmem = tmem + acc * (uint32_t)kPBN;
+      const uint32_t d_tmem = tmem + acc * (uint32_t)kDTile;
       for (int kb = 0; kb < nkb; ++kb, ++g) {
-        const int st = g % kPStages;
-        if (!mbar_wait(&s.full[st], (g / kPStages) & 1)) { s.abort_flag = 1; break; }
-        if (s.abort_flag) break;
+        const int st = g % kDStages;
+        if (!mbar_wait(&s.full[st], (g / kDStages) & 1)) { s.abort_flag = 1; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t da = make_smem_desc(smem_u32(s.a[st]));
         const uint64_t db = make_smem_desc(smem_u32(s.b[st]));
@@ -299,18 +355,18 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
           const uint64_t adv = (uint64_t)((k * kUmmaK * 4) >> 4);
           asm volatile(
               "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+              "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
               ::"r"(d_tmem), "l"(da + adv), "l"(db + adv), "r"(idesc), "r"(accumulate) : "memory");
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s.empty[st])) : "memory");
+        commit_pair(&s.empty[st]);
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&s.tfull[acc])) : "memory");
+      commit_pair(&s.tfull[acc]);
     }
   } else if (warp >= 2) {
-    // ---------------- epilogue warps
+    // ---------------- epilogue warps of both CTAs
     const int q = warp & 3;
     uint32_t it = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+    for (int t = pair; t < ntiles; t += npairs, ++it) {
       const uint32_t acc = it & 1u;
       int ok = 1;
       if (lane == 0) {
@@ -321,12 +377,12 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int m0 = (t % nbm) * kBM, n0 = (t / nbm) * kPBN;
+      const int m0 = (t % nbm) * kDTile + rank * kDHalf, n0 = (t / nbm) * kDTile;
       const int row = m0 + q * 32 + lane;
 #pragma unroll 1
-      for (int c0 = 0; c0 < kPBN; c0 += 32) {
+      for (int c0 = 0; c0 < kDTile; c0 += 32) {
         uint32_t r[32];
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + acc * (uint32_t)kPBN + (uint32_t)c0;
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + acc * (uint32_t)kDTile + (uint32_t)c0;
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
             "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -337,31 +393,13 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
               "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
             : "r"(taddr) : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c0 + 32 >= kPBN) {
-          // last chunk is in registers: hand the accumulator back to the MMA warp before the stores
+        if (c0 + 32 >= kDTile) {
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) mbar_arrive(&s.tempty[acc]);
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapa_u32(smem_u32(&s.tempty[acc]), 0)) : "memory");
         }
-        if (row < M && n0 + c0 < N) {
-          float* dst = out + (size_t)row * ldo + n0 + c0;
-          const int ncol = N - (n0 + c0);
-          if (ncol >= 32 && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              float4 v;
-              v.x = apply_act(__uint_as_float(r[j]), act);
-              v.y = apply_act(__uint_as_float(r[j + 1]), act);
-              v.z = apply_act(__uint_as_float(r[j + 2]), act);
-              v.w = apply_act(__uint_as_float(r[j + 3]), act);
-              *reinterpret_cast<float4*>(dst + j) = v;
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j < ncol) dst[j] = apply_act(__uint_as_float(r[j]), act);
-          }
-        }
+        store_chunk(r, out, out_t, row, n0 + c0, M, N, ldo, act);
       }
     }
   }
@@ -369,12 +407,55 @@ gemm_tf32_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (s.abort_flag) {
-    if (threadIdx.x == 0) set_status(status, kWaitTimeout, blockIdx.x, 200);
+    if (threadIdx.x == 0) set_status(status, kWaitTimeout, blockIdx.x, 300);
     for (int i = 0; i < 200; ++i) __nanosleep(1000);
     __syncthreads();
   }
+  cluster_sync_all();       // neither CTA frees its accumulators or leaves while the other still works
   if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------ outer products
+// The input gradient of a net's last layer, [batch, 1] · [1, in], is an outer product: no contraction for the tensor
+// cores, and a K padded to 4 takes four more launches.  The operands are cut to TF32 as the tensor cores cut them.
+__device__ __forceinline__ float tf32_cut(float x) { return __uint_as_float(__float_as_uint(x) & 0xFFFFE000u); }
+
+// K <= 4: every element is a sum of at most four products.  A thread keeps four columns' operands and walks rows.
+// Bound by writing the result: 8192x1024x1 on B200 40 -> 12 us (33 MB).
+constexpr int kRankRows = 16;
+__global__ void __launch_bounds__(256)
+k_gemm_rank4(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out, float* __restrict__ out_t, int M, int N,
+             int K, int lda, int ldb, int ldo, int act) {
+  const int n0 = (int)(blockIdx.x * 256 + threadIdx.x) * 4;
+  if (n0 >= N) return;
+  float w[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[j][k] = n0 + j < N && k < K ? tf32_cut(b[(size_t)(n0 + j) * ldb + k]) : 0.f;
+  const int m0 = blockIdx.y * kRankRows, m1 = m0 + kRankRows < M ? m0 + kRankRows : M;
+  for (int m = m0; m < m1; ++m) {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float x = k < K ? tf32_cut(a[(size_t)m * lda + k]) : 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = k < K ? v[j] + x * w[j][k] : v[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = apply_act(v[j], act);
+    float* dst = out + (size_t)m * ldo + n0;
+    if (n0 + 4 <= N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+      *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) if (n0 + j < N) dst[j] = v[j];
+    }
+    if (out_t != nullptr)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) if (n0 + j < N) out_t[(size_t)(n0 + j) * M + m] = v[j];
   }
 }
 
@@ -390,15 +471,54 @@ __global__ void k_transpose(const float* __restrict__ in, float* __restrict__ ou
   for (int j = threadIdx.y; j < 32; j += blockDim.y)
     if (c0 + j < cols && r < rows) out[(size_t)(c0 + j) * rows + r] = tile[threadIdx.x][j];
 }
+// act'(y) expressed through the activation output y
+__device__ __forceinline__ float act_slope(float yv, int act) {
+  if (act == kActRelu) return yv > 0.f ? 1.f : 0.f;
+  if (act == kActScaledTanh) { const float t = yv / 1.7159f; return 1.7159f * 0.6666667f * (1.f - t * t); }
+  if (act == kActSigmoid) return yv * (1.f - yv);
+  return 1.f;
+}
 // z = g ∘ act'(y) with act' expressed through the activation output y
 __global__ void k_act_backward(const float* __restrict__ g, const float* __restrict__ y, float* __restrict__ z, size_t n, int act) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float yv = y[i];
-    float d = 1.f;
-    if (act == kActRelu) d = yv > 0.f ? 1.f : 0.f;
-    else if (act == kActScaledTanh) { const float t = yv / 1.7159f; d = 1.7159f * 0.6666667f * (1.f - t * t); }
-    else if (act == kActSigmoid) d = yv * (1.f - yv);
-    z[i] = g[i] * d;
+    z[i] = g[i] * act_slope(y[i], act);
+  }
+}
+// z = g ∘ act'(y) (unless null) and its transpose in one pass over g and y: the weight gradient needs zᵀ, the
+// input gradient z.  64 x 64 tiles: 16-byte global accesses both ways where rows and columns are multiples of 4
+// (kVec), one float at a time otherwise; the tile's odd row length keeps the transposed reads free of bank conflicts.
+constexpr int kActTile = 64;
+template <bool kVec>
+__global__ void __launch_bounds__(256)
+k_act_backward_t(const float* __restrict__ g, const float* __restrict__ y, float* __restrict__ z, float* __restrict__ zt, int rows,
+                 int cols, int act) {
+  __shared__ float tile[kActTile][kActTile + 1];
+  const int r0 = blockIdx.y * kActTile, c0 = blockIdx.x * kActTile;
+  constexpr int kW = kVec ? 4 : 1, kLine = kActTile / kW;
+  for (int i = threadIdx.x; i < kActTile * kLine; i += 256) {
+    const int r = i / kLine, c = (i % kLine) * kW;
+    if (r0 + r >= rows || c0 + c >= cols) continue;
+    const size_t at = (size_t)(r0 + r) * cols + c0 + c;
+    if (kVec) {
+      const float4 gv = *reinterpret_cast<const float4*>(g + at), yv = *reinterpret_cast<const float4*>(y + at);
+      float4 v;
+      v.x = gv.x * act_slope(yv.x, act); v.y = gv.y * act_slope(yv.y, act);
+      v.z = gv.z * act_slope(yv.z, act); v.w = gv.w * act_slope(yv.w, act);
+      if (z != nullptr) *reinterpret_cast<float4*>(z + at) = v;
+      tile[r][c] = v.x; tile[r][c + 1] = v.y; tile[r][c + 2] = v.z; tile[r][c + 3] = v.w;
+    } else {
+      const float v = g[at] * act_slope(y[at], act);
+      if (z != nullptr) z[at] = v;
+      tile[r][c] = v;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kActTile * kLine; i += 256) {
+    const int c = i / kLine, r = (i % kLine) * kW;
+    if (r0 + r >= rows || c0 + c >= cols) continue;
+    float* dst = zt + (size_t)(c0 + c) * rows + r0 + r;
+    if (kVec) *reinterpret_cast<float4*>(dst) = make_float4(tile[r][c], tile[r + 1][c], tile[r + 2][c], tile[r + 3][c]);
+    else *dst = tile[r][c];
   }
 }
 // logistic loss layer: loss += Σ log(1+e^{-x y}); grad = -y/(1+e^{x y})   (src/neural_network/loss_layer.h:39-58)
@@ -468,7 +588,7 @@ EncodeTiledFn get_encode() {
   return fn;
 }
 // 2-D map over a row-major [rows, k] fp32 matrix with row stride ld (floats), box = 128 rows x 32 floats, 128B swizzle
-int make_map(CUtensorMap* map, const float* base, int rows, int k, int ld, int box_rows = kBM) {
+int make_map(CUtensorMap* map, const float* base, int rows, int k, int ld, int box_rows) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return -1;
   const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
@@ -480,52 +600,69 @@ int make_map(CUtensorMap* map, const float* base, int rows, int k, int ld, int b
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
+// 256x256 tiles from which on CTA pairs are faster than one 128x128 tile per CTA: 2048x1024x2048 (32 tiles) takes 31 us in
+// tiles and 41 in pairs, 2048x2048x512 (64 tiles) 34 and 27
+constexpr long kPairTiles = 48;
+template <int kRows, int kCols>
+int launch_tile(const float* a, const float* b, float* out, float* out_t, int M, int N, int K, int lda, int ldb, int ldo, int act,
+                uint32_t* status, cudaStream_t stream) {
+  CUtensorMap ma, mb;
+  int r = make_map(&ma, a, M, K, lda, kRows);
+  if (r == 0) r = make_map(&mb, b, N, K, ldb, kCols);
+  if (r) return r;
+  const size_t smem = sizeof(GemmSmem) + 1024;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tf32_tcgen05_kernel<kRows, kCols>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  const dim3 grid((M + kBM - 1) / kBM, (N + kCols - 1) / kCols);
+  gemm_tf32_tcgen05_kernel<kRows, kCols><<<grid, 128, smem, stream>>>(ma, mb, out, out_t, M, N, K, ldo, act, status);
+  return (int)cudaGetLastError();
+}
 inline int egrid(size_t n) { size_t b = (n + 255) / 256; if (b < 1) b = 1; if (b > 148 * 8) b = 148 * 8; return (int)b; }
 
 }  // namespace
 
 extern "C" {
 
-// out[M,N] (row stride ldo) = act(a[M,K] (row stride lda) · b[N,K]ᵀ (row stride ldb)).
-// Requirements: a, b 16-byte aligned; lda, ldb multiples of 4 floats.  Returns 0, a CUDA error, or
+// out[M,N] (row stride ldo) = act(a[M,K] (row stride lda) · b[N,K]ᵀ (row stride ldb)); out_t, when not null,
+// receives the transpose [N,M] too.  variant: 0 by size, 1 one tile per CTA, 2 CTA pairs, 3 K of at most four.
+// Requirements: a, b 16-byte aligned; lda, ldb multiples of 4 floats (variant 3: none).  Returns 0, a CUDA error, or
 // -1 when tensor maps cannot be created (no driver entry point).
-int psb_gemm_tn_tf32(const float* a, const float* b, float* out, int M, int N, int K, int lda, int ldb, int ldo, int act,
-                     uint32_t* status, cudaStream_t stream) {
+int psb_gemm_tn_tf32(const float* a, const float* b, float* out, float* out_t, int M, int N, int K, int lda, int ldb, int ldo, int act,
+                     int variant, uint32_t* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((lda & 3) || (ldb & 3) || (reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15)) return (int)cudaErrorInvalidValue;
-  CUtensorMap ma, mb;
-  int r = make_map(&ma, a, M, K, lda);
-  if (r) return r;
-  // large problems: persistent kernel with 128x256 tiles and a double-buffered accumulator
-  static int sms = 0;
-  if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-  const long tiles_p = (long)((M + kBM - 1) / kBM) * ((N + kPBN - 1) / kPBN);
-  if (tiles_p >= sms) {
-    r = make_map(&mb, b, N, K, ldb, kPBN);
-    if (r) return r;
-    const size_t smem_p = sizeof(GemmSmemP) + 1024;
-    static bool attr_p = false;
-    if (!attr_p) {
-      cudaError_t e = cudaFuncSetAttribute(gemm_tf32_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p);
-      if (e != cudaSuccess) return (int)e;
-      attr_p = true;
-    }
-    const int grid = (int)(tiles_p < sms ? tiles_p : sms);
-    gemm_tf32_persistent_kernel<<<grid, kPThreads, smem_p, stream>>>(ma, mb, out, M, N, K, ldo, act, status);
+  const bool aligned = ((lda | ldb) & 3) == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
+  if (variant == 3 ? K > 4 : !aligned) return (int)cudaErrorInvalidValue;
+  const dim3 rank_grid((N + 1023) / 1024, (M + kRankRows - 1) / kRankRows);
+  const long tiles_d = (long)((M + kDTile - 1) / kDTile) * ((N + kDTile - 1) / kDTile);
+  if (variant == 0) variant = K <= 4 && rank_grid.y < 65536u ? 3 : tiles_d >= kPairTiles ? 2 : 1;
+  if (variant == 3) {
+    k_gemm_rank4<<<rank_grid, 256, 0, stream>>>(a, b, out, out_t, M, N, K, lda, ldb, ldo, act);
     return (int)cudaGetLastError();
   }
-  r = make_map(&mb, b, N, K, ldb);
-  if (r) return r;
-  const size_t smem = sizeof(GemmSmem) + 1024;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tf32_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
+  if (variant == 2) {
+    CUtensorMap ma, mb;
+    int r = make_map(&ma, a, M, K, lda, kDHalf);
+    if (r == 0) r = make_map(&mb, b, N, K, ldb, kDHalf);
+    if (r) return r;
+    static int sms = 0;
+    if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+    const size_t smem_d = sizeof(GemmSmemD) + 1024;
+    static bool attr_d = false;
+    if (!attr_d) {
+      cudaError_t e = cudaFuncSetAttribute(gemm_tf32_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_d);
+      if (e != cudaSuccess) return (int)e;
+      attr_d = true;
+    }
+    const int pairs = (int)(tiles_d < sms / 2 ? tiles_d : sms / 2);
+    gemm_tf32_pair_kernel<<<2 * pairs, kPThreads, smem_d, stream>>>(ma, mb, out, out_t, M, N, K, ldo, act, status);
+    return (int)cudaGetLastError();
   }
-  dim3 grid((M + kBM - 1) / kBM, (N + kBN - 1) / kBN);
-  gemm_tf32_tcgen05_kernel<<<grid, 128, smem, stream>>>(ma, mb, out, M, N, K, ldo, act, status);
-  return (int)cudaGetLastError();
+  if (M <= kThinRows) return launch_tile<kThinRows, kThinCols>(a, b, out, out_t, M, N, K, lda, ldb, ldo, act, status, stream);
+  return launch_tile<kBM, kBN>(a, b, out, out_t, M, N, K, lda, ldb, ldo, act, status, stream);
 }
 int psb_transpose(const float* in, float* out, int rows, int cols, cudaStream_t s) {
   dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
@@ -534,6 +671,16 @@ int psb_transpose(const float* in, float* out, int rows, int cols, cudaStream_t 
 }
 int psb_act_backward(const float* g, const float* y, float* z, size_t n, int act, cudaStream_t s) {
   k_act_backward<<<egrid(n), 256, 0, s>>>(g, y, z, n, act);
+  return (int)cudaGetLastError();
+}
+// z (may be null) and its transpose zt [cols, rows]
+int psb_act_backward_t(const float* g, const float* y, float* z, float* zt, int rows, int cols, int act, cudaStream_t s) {
+  if (rows <= 0 || cols <= 0) return 0;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(zt);
+  const dim3 grid((cols + kActTile - 1) / kActTile, (rows + kActTile - 1) / kActTile);
+  if (grid.y > 65535u) return (int)cudaErrorInvalidValue;
+  if (((rows | cols) & 3) == 0 && (all & 15) == 0) k_act_backward_t<true><<<grid, 256, 0, s>>>(g, y, z, zt, rows, cols, act);
+  else k_act_backward_t<false><<<grid, 256, 0, s>>>(g, y, z, zt, rows, cols, act);
   return (int)cudaGetLastError();
 }
 int psb_logistic_loss(const float* x, const float* y, float* grad, size_t n, double* loss, cudaStream_t s) {

@@ -164,13 +164,22 @@ class FullyConnectedLayer(Layer):
         x = self.inputs[0].value
         self._ensure_model(x.shape[1])
         self.x = x
-        self.outputs[0].value = dense.gemm_tn(x, self.model.value, self.act, pad_k=True)
+        out = self.outputs[0]
+        # a dense layer that reads this edge needs its transpose for the weight gradient: the GEMM writes both
+        yt = torch.empty((self.out_dim, x.shape[0]), dtype=torch.float32, device=x.device) \
+            if self.net.training and out.read_by_dense else None
+        out.value = dense.gemm_tn(x, self.model.value, self.act, pad_k=True, out_t=yt)
+        out.transposed = None if yt is None else (out.value, out.value._version, yt)
         return 0.0
 
     def backward(self) -> None:
         y, gy = self.outputs[0].value, self.outputs[0].gradient
-        z = gy if self.act == "IDENTITY" else dense.act_backward(gy, y, self.act)
-        zt, xt = dense.transpose(z), dense.transpose(self.x)
+        if self.act == "IDENTITY":
+            z, zt = gy, dense.transpose(gy)
+        else:
+            z, zt = dense.act_backward_t(gy, y, self.act, want_z=self.inputs[0].needs_grad)
+        t, self.inputs[0].transposed = self.inputs[0].transposed, None
+        xt = t[2] if t is not None and t[0] is self.x and t[0]._version == t[1] else dense.transpose(self.x)
         self.model.gradient = dense.gemm_tn(zt, xt, pad_k=True)                       # [out, in] = Zᵀ · X
         if self.inputs[0].needs_grad:
             wt = dense.transpose(self.model.value)                        # [in, out]
@@ -239,6 +248,8 @@ LAYERS = {"DATA": DataLayer, "FULLY_CONNECTED": FullyConnectedLayer, "SPARSE_FUL
 
 class Edge(Parameter):
     needs_grad: bool = True
+    read_by_dense: bool = False                  # a fully connected layer has this edge as its input
+    transposed: Optional[tuple] = None           # (value, its version, valueᵀ) from the layer that wrote the value
 
 
 class Net:
@@ -255,6 +266,8 @@ class Net:
             self.layers.append(LAYERS[lc.type](lc, self))
         for l in self.layers:
             l.init()
+            if isinstance(l, FullyConnectedLayer):
+                l.inputs[0].read_by_dense = True
             if isinstance(l, DataLayer):
                 for e in l.outputs:
                     e.needs_grad = False

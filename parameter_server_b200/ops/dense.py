@@ -29,13 +29,17 @@ def check_status(dev) -> None:
 
 
 def gemm_tn(a: torch.Tensor, b: torch.Tensor, act: str = "IDENTITY", out: Optional[torch.Tensor] = None,
-            pad_k: bool = False) -> torch.Tensor:
-    """``act(a @ b.T)`` for row-major fp32 ``a`` [M,K] and ``b`` [N,K] on the tcgen05 tensor cores (TF32)."""
+            pad_k: bool = False, out_t: Optional[torch.Tensor] = None, variant: int = 0) -> torch.Tensor:
+    """``act(a @ b.T)`` for row-major fp32 ``a`` [M,K] and ``b`` [N,K] on the tcgen05 tensor cores (TF32).  ``out_t``
+    (contiguous [N,M]) receives the transposed result too; ``variant``: 0 = kernel by size, 1 = one tile per thread
+    block, 2 = pairs of thread blocks, 3 = a K of at most four."""
     assert a.is_cuda and a.dtype == torch.float32 and b.dtype == torch.float32 and a.shape[1] == b.shape[1]
     assert a.stride(1) == 1 and b.stride(1) == 1
     M, K = a.shape
     Nn = b.shape[0]
-    if pad_k and K % 4:
+    if pad_k and K < 4 and variant == 0:
+        variant = 3                                  # reads the operands element by element
+    elif pad_k and K % 4:
         # TMA needs row strides that are multiples of 16 bytes: zero-pad the contraction dimension
         kp = (K + 3) // 4 * 4
         a = torch.nn.functional.pad(a, (0, kp - K))
@@ -43,8 +47,10 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor, act: str = "IDENTITY", out: Option
         K = kp
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.float32, device=a.device)
-    rc = N.lib().psb_gemm_tn_tf32(N.ptr(a), N.ptr(b), N.ptr(out), M, Nn, K, a.stride(0), b.stride(0), out.stride(0), ACT[act],
-                                  N.ptr(_status_for(a.device)), N.stream_ptr())
+    if out_t is not None:
+        assert out_t.shape == (Nn, M) and out_t.is_contiguous() and out_t.dtype == torch.float32
+    rc = N.lib().psb_gemm_tn_tf32(N.ptr(a), N.ptr(b), N.ptr(out), N.ptr(out_t), M, Nn, K, a.stride(0), b.stride(0), out.stride(0),
+                                  ACT[act], variant, N.ptr(_status_for(a.device)), N.stream_ptr())
     if rc == 1:
         raise ValueError("gemm_tn needs 16-byte aligned operands whose row strides are multiples of 4 floats")
     N.check(rc, "gemm_tn_tf32")
@@ -62,6 +68,16 @@ def act_backward(g: torch.Tensor, y: torch.Tensor, act: str) -> torch.Tensor:
     z = torch.empty_like(g)
     N.check(N.lib().psb_act_backward(N.ptr(g), N.ptr(y), N.ptr(z), C.c_size_t(g.numel()), ACT[act], N.stream_ptr()), "act_backward")
     return z
+
+
+def act_backward_t(g: torch.Tensor, y: torch.Tensor, act: str, want_z: bool = True):
+    """(``g ∘ act'(y)`` or None, its transpose) of two contiguous [rows, cols] matrices in one pass over them."""
+    assert g.is_contiguous() and y.is_contiguous() and g.shape == y.shape and g.dim() == 2
+    z = torch.empty_like(g) if want_z else None
+    zt = torch.empty((g.shape[1], g.shape[0]), dtype=torch.float32, device=g.device)
+    N.check(N.lib().psb_act_backward_t(N.ptr(g), N.ptr(y), N.ptr(z), N.ptr(zt), g.shape[0], g.shape[1], ACT[act], N.stream_ptr()),
+            "act_backward_t")
+    return z, zt
 
 
 def logistic_loss(x: torch.Tensor, y: torch.Tensor, want_grad: bool = True):

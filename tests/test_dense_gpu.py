@@ -16,7 +16,7 @@ def _ref_act(x, act):
 
 
 @pytest.mark.parametrize("M,N,K", [(128, 128, 32), (128, 128, 256), (256, 384, 96), (200, 130, 72), (1000, 520, 1024), (64, 8, 4),
-                                   # >= 148 tiles of 128x256: the persistent kernel (several tiles per CTA, ragged edges, short K)
+                                   # many tiles: persistent CTA pairs (several tiles per pair, ragged edges, short K)
                                    (2048, 4096, 512), (1925, 2563, 260), (4096, 4224, 36), (9000, 2100, 64)])
 @pytest.mark.parametrize("act", ["IDENTITY", "RELU", "SCALED_TANH"])
 def test_gemm_tn_matches_fp32(M, N, K, act):
@@ -35,6 +35,55 @@ def test_gemm_tn_matches_fp32(M, N, K, act):
     err = (out - ref).abs().max().item()
     assert err < 2e-2 * max(1.0, ref.abs().max().item()), err        # TF32: 10-bit mantissa
     assert (out - ref).abs().mean().item() < 2e-3
+
+
+@pytest.mark.parametrize("M,N,K,variant", [
+    (256, 256, 32, 2), (257, 255, 36, 2), (5, 2000, 64, 2), (130, 120, 200, 2), (5000, 1300, 132, 2),     # CTA pairs
+    (128, 128, 28, 1), (129, 127, 220, 1), (7, 9, 700, 1),                                                # one tile per CTA
+    (1, 1000, 2052, 0), (8, 32, 32, 0), (9, 33, 64, 0), (3, 130, 36, 0), (8, 31, 5000, 0), (1, 1, 8, 0),       # few rows
+    (100, 203, 1, 0), (37, 1, 3, 0), (1, 64, 2, 0), (1030, 5, 4, 0)])                                     # K of at most four
+@pytest.mark.parametrize("act", ["IDENTITY", "SIGMOID"])
+def test_gemm_kernels_and_transposed_result(M, N, K, variant, act):
+    """Every kernel at the edges of its tiles against fp64: TF32 operands carry a relative error below 2^-10 each, so
+    an element is off by at most 2^-9 of the sum of its terms' magnitudes (plus the fp32 sums, far below)."""
+    from parameter_server_b200.ops import dense
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a, b = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda") / K ** 0.5
+    t = torch.full((N, M), float("nan"), device="cuda")
+    out = dense.gemm_tn(a, b, act, pad_k=True, out_t=t, variant=variant)
+    torch.cuda.synchronize()
+    dense.check_status(a.device)
+    ref, bound = a.double() @ b.double().T, (a.double().abs() @ b.double().abs().T) / 512 + 1e-5
+    if act == "SIGMOID":
+        ref, bound = torch.sigmoid(ref), bound / 4 + 1e-5
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    assert torch.equal(t, out.T)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 8192), (8, 96, 260), (700, 900, 520)])
+def test_kernels_agree_to_the_bit(M, N, K):
+    """Which kernel a product's size selects does not change its sums: the tile kernels add in the same order, and the
+    outer product cuts its operands to TF32 as the tensor cores do."""
+    from parameter_server_b200.ops import dense
+
+    a, b = torch.randn(M, K, device="cuda"), torch.randn(N, K, device="cuda")
+    assert torch.equal(dense.gemm_tn(a, b), dense.gemm_tn(a, b, variant=2))
+    a, b = torch.nn.functional.pad(a[:, :1], (0, 3)), torch.nn.functional.pad(b[:, :1], (0, 3))
+    assert torch.equal(dense.gemm_tn(a, b, variant=3), dense.gemm_tn(a, b, variant=2))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (64, 64), (63, 65), (128, 4), (70, 200), (333, 77)])
+@pytest.mark.parametrize("act", ["RELU", "SCALED_TANH", "SIGMOID"])
+def test_act_backward_with_transpose(rows, cols, act):
+    from parameter_server_b200.ops import dense
+
+    y, g = torch.rand(rows, cols, device="cuda") - 0.3, torch.randn(rows, cols, device="cuda")
+    want = dense.act_backward(g, y, act)
+    z, zt = dense.act_backward_t(g, y, act)
+    assert torch.equal(z, want) and torch.equal(zt, want.T)
+    z, zt = dense.act_backward_t(g, y, act, want_z=False)
+    assert z is None and torch.equal(zt, want.T)
 
 
 def test_gemm_strided_views_and_repeat():
