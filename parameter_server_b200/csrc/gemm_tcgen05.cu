@@ -471,6 +471,30 @@ __global__ void k_transpose(const float* __restrict__ in, float* __restrict__ ou
   for (int j = threadIdx.y; j < 32; j += blockDim.y)
     if (c0 + j < cols && r < rows) out[(size_t)(c0 + j) * rows + r] = tile[threadIdx.x][j];
 }
+// A minibatch in one launch: rows sel[] of x, their labels, and (unless null) the transposed rows that the first
+// layer's weight gradient reads.  For 256 rows of 64 floats the three index and transpose launches it stands for are
+// host time.
+__global__ void k_gather_minibatch(const float* __restrict__ x, const float* __restrict__ y, const int64_t* __restrict__ sel, int rows,
+                                   int cols, float* __restrict__ xb, float* __restrict__ xbt, float* __restrict__ yb) {
+  __shared__ float tile[32][33];
+  const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    const int r = r0 + j;
+    if (r >= rows) continue;
+    const size_t from = (size_t)sel[r];
+    if (c < cols) {
+      const float v = x[from * cols + c];
+      xb[(size_t)r * cols + c] = v;
+      tile[j][threadIdx.x] = v;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) yb[r] = y[from];
+  }
+  if (xbt == nullptr) return;
+  __syncthreads();
+  const int r = r0 + threadIdx.x, c0 = blockIdx.x * 32;
+  for (int j = threadIdx.y; j < 32; j += blockDim.y)
+    if (c0 + j < cols && r < rows) xbt[(size_t)(c0 + j) * rows + r] = tile[threadIdx.x][j];
+}
 // act'(y) expressed through the activation output y
 __device__ __forceinline__ float act_slope(float yv, int act) {
   if (act == kActRelu) return yv > 0.f ? 1.f : 0.f;
@@ -667,6 +691,15 @@ int psb_gemm_tn_tf32(const float* a, const float* b, float* out, float* out_t, i
 int psb_transpose(const float* in, float* out, int rows, int cols, cudaStream_t s) {
   dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
   k_transpose<<<grid, block, 0, s>>>(in, out, rows, cols);
+  return (int)cudaGetLastError();
+}
+// sel: rows indices into x [*, cols] and y; xbt may be null
+int psb_gather_minibatch(const float* x, const float* y, const int64_t* sel, int rows, int cols, float* xb, float* xbt, float* yb,
+                         cudaStream_t s) {
+  if (rows <= 0 || cols <= 0) return 0;
+  const dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
+  if (grid.y > 65535u) return (int)cudaErrorInvalidValue;
+  k_gather_minibatch<<<grid, block, 0, s>>>(x, y, sel, rows, cols, xb, xbt, yb);
   return (int)cudaGetLastError();
 }
 int psb_act_backward(const float* g, const float* y, float* z, size_t n, int act, cudaStream_t s) {

@@ -131,11 +131,20 @@ class DataLayer(Layer):
         else:
             b -= b % 4        # GEMM operand strides are multiples of 4 floats
             sel = torch.randperm(n, generator=self.gen)[:b].to(self.net.device)
-            xb, yb = self.X[sel].contiguous(), self.y[sel].contiguous()
+            if self.X.is_cuda and self.y.is_contiguous() and b <= 32 * 65535:
+                xb, xbt, yb = dense.gather_minibatch(self.X, self.y, sel, self.net.training and self.outputs[0].read_by_dense)
+                self.outputs[0].transposed = None if xbt is None else (xb, xb._version, xbt)
+            else:
+                xb, yb = self.X[sel].contiguous(), self.y[sel].contiguous()
         self.outputs[0].value = xb
         if len(self.outputs) > 1:
             self.outputs[1].value = yb
         return 0.0
+
+
+def _transposed(x: torch.Tensor) -> torch.Tensor:
+    """``xᵀ``, contiguous, to be read only: a single row or column is laid out like its transpose."""
+    return x.reshape(x.shape[1], x.shape[0]) if 1 in x.shape and x.is_contiguous() else dense.transpose(x)
 
 
 class FullyConnectedLayer(Layer):
@@ -175,14 +184,14 @@ class FullyConnectedLayer(Layer):
     def backward(self) -> None:
         y, gy = self.outputs[0].value, self.outputs[0].gradient
         if self.act == "IDENTITY":
-            z, zt = gy, dense.transpose(gy)
+            z, zt = gy, _transposed(gy)
         else:
             z, zt = dense.act_backward_t(gy, y, self.act, want_z=self.inputs[0].needs_grad)
         t, self.inputs[0].transposed = self.inputs[0].transposed, None
-        xt = t[2] if t is not None and t[0] is self.x and t[0]._version == t[1] else dense.transpose(self.x)
+        xt = t[2] if t is not None and t[0] is self.x and t[0]._version == t[1] else _transposed(self.x)
         self.model.gradient = dense.gemm_tn(zt, xt, pad_k=True)                       # [out, in] = Zᵀ · X
         if self.inputs[0].needs_grad:
-            wt = dense.transpose(self.model.value)                        # [in, out]
+            wt = _transposed(self.model.value)                            # [in, out]
             self.inputs[0].gradient = dense.gemm_tn(z, wt, pad_k=True)                # [batch, in] = Z · W
 
 

@@ -80,6 +80,19 @@ def act_backward_t(g: torch.Tensor, y: torch.Tensor, act: str, want_z: bool = Tr
     return z, zt
 
 
+def gather_minibatch(x: torch.Tensor, y: torch.Tensor, sel: torch.Tensor, want_t: bool):
+    """(``x[sel]``, its transpose or None, ``y[sel]``) for contiguous float32 ``x`` [n, cols], ``y`` [n] and device
+    int64 row numbers ``sel`` (all inside x), in one launch."""
+    assert x.is_contiguous() and y.is_contiguous() and sel.is_contiguous() and x.dtype == y.dtype == torch.float32 and sel.dtype == torch.int64
+    b, cols = sel.numel(), x.shape[1]
+    xb = torch.empty((b, cols), dtype=torch.float32, device=x.device)
+    yb = torch.empty(b, dtype=torch.float32, device=x.device)
+    xbt = torch.empty((cols, b), dtype=torch.float32, device=x.device) if want_t else None
+    N.check(N.lib().psb_gather_minibatch(N.ptr(x), N.ptr(y), N.ptr(sel), b, cols, N.ptr(xb), N.ptr(xbt), N.ptr(yb), N.stream_ptr()),
+            "gather_minibatch")
+    return xb, xbt, yb
+
+
 def logistic_loss(x: torch.Tensor, y: torch.Tensor, want_grad: bool = True):
     """(Σ log(1+e^{-x·y}) as a 1-element fp64 tensor, −y/(1+e^{x·y}) or None)."""
     loss = torch.zeros(1, dtype=torch.float64, device=x.device)

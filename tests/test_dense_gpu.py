@@ -132,3 +132,16 @@ def test_elementwise_kernels():
     dense.col_normalize(m)
     torch.testing.assert_close(m.mean(0), torch.zeros(9, device="cuda"), atol=1e-5, rtol=0)
     torch.testing.assert_close(m.norm(dim=0), torch.full((9,), 200 ** 0.5, device="cuda"), rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("rows,cols,b", [(1, 1, 1), (100, 3, 37), (500, 64, 256), (70, 33, 33), (4000, 129, 100)])
+def test_gather_minibatch(rows, cols, b):
+    from parameter_server_b200.ops import dense
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, y = torch.randn(rows, cols, generator=g, device="cuda"), torch.randn(rows, generator=g, device="cuda")
+    sel = torch.randint(0, rows, (b,), generator=g, device="cuda")
+    for want_t in (True, False):
+        xb, xbt, yb = dense.gather_minibatch(x, y, sel, want_t)
+        assert torch.equal(xb, x[sel]) and torch.equal(yb, y[sel])
+        assert torch.equal(xbt, x[sel].T) if want_t else xbt is None
