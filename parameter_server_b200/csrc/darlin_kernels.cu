@@ -33,6 +33,7 @@
 // records the place in the status word, raises the abort flag and every CTA leaves the
 // block loop.
 #include <cstdlib>
+#include <mutex>
 
 #include "reduce_kernels.cuh"
 
@@ -1425,11 +1426,9 @@ constexpr int64_t kSoloClusterNnz = 14336;
 
 struct SoloPlan { int sms = 0, cluster = 0; };
 
-// SMs of the current device and the largest cluster of the kernel it can hold (16 thread blocks, else 8; 0: none)
-SoloPlan solo_plan(const void* cluster_kernel) {
+// SMs of a device and the largest cluster of the kernel it can hold (16 thread blocks, else 8; 0: none)
+SoloPlan make_solo_plan(const void* cluster_kernel, int dev) {
   SoloPlan p;
-  int dev = 0;
-  cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev);
   if (cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
   for (int c = 16; c >= 8 && p.cluster == 0; c >>= 1) {
@@ -1446,13 +1445,26 @@ SoloPlan solo_plan(const void* cluster_kernel) {
   return p;
 }
 
+// ... of the current device, asked for once
+SoloPlan solo_plan(const void* cluster_kernel, bool vals) {
+  static std::mutex lock;
+  static SoloPlan known[2][16];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) return make_solo_plan(cluster_kernel, dev);
+  std::lock_guard<std::mutex> g(lock);
+  SoloPlan& p = known[vals ? 1 : 0][dev];
+  if (p.sms == 0) p = make_solo_plan(cluster_kernel, dev);
+  return p;
+}
+
 int solo_launch(const DarlinWorker& Wk, const DarlinPeers& P, const DarlinServer& S, const DarlinSched& Q, const DarlinHyper& H,
                 cudaStream_t stream) {
   DarlinWorker w = Wk; DarlinPeers p = P; DarlinServer s = S; DarlinSched q = Q; DarlinHyper h = H;
   void* args[] = {&w, &p, &s, &q, &h};
   const void* cl = w.vals != nullptr ? (const void*)darlin_solo_kernel<true, true> : (const void*)darlin_solo_kernel<true, false>;
   const void* gr = w.vals != nullptr ? (const void*)darlin_solo_kernel<false, true> : (const void*)darlin_solo_kernel<false, false>;
-  const SoloPlan plan = solo_plan(cl);
+  const SoloPlan plan = solo_plan(cl, w.vals != nullptr);
   const bool cluster = plan.cluster > 0 && (q.variant == 2 || (q.variant == 0 && q.group_nnz <= kSoloClusterNnz));
   if (!cluster) return (int)cudaLaunchCooperativeKernel(gr, dim3((unsigned)plan.sms), dim3(kSoloThreads), args, 0, stream);
   cudaLaunchConfig_t cfg{};
