@@ -899,8 +899,10 @@ ftrl_pull_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_
   }
 }
 
-// A training step, whole (kPull) or after ftrl_pull_kernel: rows and push.
-constexpr int kStepBlocksPerSM = 5, kPushBlocksPerSM = 6;
+// A training step, whole (kPull) or after ftrl_pull_kernel: rows and push.  Rows and push alone: 100,000 rows with
+// 3 / 4 / 5 / 6 blocks per SM take 657 / 639 / 656 / 676 us a step (count rule), 690 / 580 / 590 / 600 (sum of squares);
+// from 5 on registers spill, with 3 too few random accesses are in flight.  Whole, 4 and 5 measure the same.
+constexpr int kStepBlocksPerSM = 5, kPushBlocksPerSM = 4;
 template <bool kCounts, bool kPull>
 __global__ void __launch_bounds__(256, kPull ? kStepBlocksPerSM : kPushBlocksPerSM)
 ftrl_step_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t pull_seq, uint32_t push_seq, uint32_t flags,
@@ -1153,8 +1155,8 @@ int psb_ftrl_pull_spmv(const FtrlPeers* P, const Minibatch* M, const LocalScratc
 }
 
 // Non-zeros from which on a step takes two launches: the pull gains more from its own 8 blocks per SM than the second
-// launch costs.  B200, step in one / two launches (count rule): 48 k non-zeros 44 / 48 us, 1 M 185 / 190, 2.9 M 325 / 315,
-// 5.3 M 432 / 419, 9.6 M 738 / 670.
+// launch costs.  B200, step in one / two launches (count rule, 6 blocks per SM in the second): 48 k non-zeros 44 / 48 us,
+// 1 M 185 / 190, 2.9 M 325 / 315, 5.3 M 432 / 419, 9.6 M 738 / 670.
 constexpr int64_t kTwoLaunchNnz = 1500000;
 
 // One training step: pull, rows, push (sequence numbers of the pull's and the push's flags).  flags bit 0: create

@@ -150,11 +150,15 @@ def test_minibatches_of_changing_size_and_one_without_repeated_keys(rule):
 
 @pytest.mark.parametrize("valued", [False, True])
 @pytest.mark.parametrize("rule", ["count", "sumsq"])
-def test_rows_of_all_lengths(rule, valued):
-    """Rows without non-zeros, around one warp and around what a warp keeps in registers, and far longer ones."""
+@pytest.mark.parametrize("launches,log2", [(1, 16), (2, 16), (2, 23)])
+def test_rows_of_all_lengths(rule, valued, launches, log2):
+    """Rows without non-zeros, around one warp and around what a warp keeps in registers, and far longer ones; in one
+    and in two launches, and with more slots (2^23) than a packed slot reference can tell."""
     from parameter_server_b200.models.ftrl import DeviceMinibatch
 
-    eng, hy = _engine(rule=rule)
+    eng, hy = _engine(rule=rule, local_capacity=1 << log2, table_capacity=1 << 18)
+    eng._L.two_launch_nnz = 1 if launches == 2 else 1 << 60
+    eng.region[1] = log2 if log2 > 22 else 0
     ref = FTRLRef(hy.alpha, hy.beta, hy.lambda1, hy.lambda2, rule)
     rng = np.random.RandomState(4)
     for lens in ([0], [1], [0, 1, 31, 32, 33, 0, 127, 128, 129, 160, 1000, 0], [5] * 3000, [129] * 17):
