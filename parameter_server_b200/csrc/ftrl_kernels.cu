@@ -440,7 +440,7 @@ __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScra
 constexpr int kRowBatch = 4;
 
 __device__ __forceinline__ void phase_spmv_loss(const Minibatch& M, const LocalScratch& L, const Refs refs, size_t gwarp,
-                                                size_t nwarps, int lane) {
+                                                size_t nwarps, int lane, bool count) {
   double loss = 0.0;
   PSB_STREAM_POLICY(pol);
   for (int64_t row = (int64_t)gwarp; row < M.rows; row += (int64_t)nwarps) {
@@ -469,7 +469,7 @@ __device__ __forceinline__ void phase_spmv_loss(const Minibatch& M, const LocalS
       L.xw[row] = s;
     }
   }
-  block_add1(L.stats, 0, loss);      // (lane 0 has the row's loss, the others zero)
+  if (count) block_add1(L.stats, 0, loss);      // (lane 0 has the row's loss, the others zero)
 }
 
 // Block-local cache of gradient accumulators for frequently hit slots.  Under Zipf
@@ -833,7 +833,7 @@ __device__ __forceinline__ void phase_apply_filtered(cg::grid_group& grid, const
 
 // ------------------------------------------------------------ fused kernels
 constexpr uint32_t kPullInsert = 1u;   // flags: create missing keys in the shard
-constexpr uint32_t kPullRows = 2u;     // ftrl_pull_kernel: multiply the rows too
+constexpr uint32_t kPullPredict = 2u;  // ftrl_pull_kernel: a prediction
 
 // De-duplication and lookup: the table is complete, every owner has been told, this rank's owner side has served
 // every worker, and every owner has served this one.  Returns the log2 slots worked in.
@@ -854,7 +854,7 @@ __device__ __forceinline__ uint32_t pull_weights(cg::grid_group& grid, const Ftr
     grid.sync();
     if (gtid == 0) L.region[kRegionFloor] = rlog2;    // a size that did not fit is never tried again
   }
-  block_add1(L.stats, 5, (double)fresh);
+  if (!(flags & kPullPredict)) block_add1(L.stats, 5, (double)fresh);
   if (gtid == 0) L.region[kRegionNow] = rlog2;
   PSB_TRACE(L, gtid, 1);
   // this worker's table is complete: tell every owner, then serve the other workers' tables
@@ -881,7 +881,9 @@ __device__ __forceinline__ uint32_t pull_weights(cg::grid_group& grid, const Ftr
   return rlog2;
 }
 
-// The pull on its own: of a prediction (with X·w), and of a large training step.  8 blocks of 256 threads per SM (32
+// The pull on its own: of a large training step, and of a prediction, which also multiplies the rows, empties the
+// key table again (every owner has replied, nobody reads it any more) and leaves the statistics alone: one launch
+// where saving and restoring them and emptying the table took four more.  8 blocks of 256 threads per SM (32
 // registers per thread): its phases are bound by memory latency and speed up with every resident warp.
 constexpr int kPullBlocksPerSM = 8;
 __global__ void __launch_bounds__(256, kPullBlocksPerSM)
@@ -890,11 +892,13 @@ ftrl_pull_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t gsz = (size_t)gridDim.x * blockDim.x;
   __shared__ int sh_ok;
-  if (gtid == 0) L.stats[1] += (double)M.rows;
+  const bool predict = (flags & kPullPredict) != 0u;
+  if (gtid == 0 && !predict) L.stats[1] += (double)M.rows;
   PSB_TRACE(L, gtid, 0);
   const uint32_t rlog2 = pull_weights<1>(grid, P, M, L, seq, flags, try_log2, gtid, gsz, &sh_ok);
-  if (flags & kPullRows) {
-    phase_spmv_loss(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, threadIdx.x & 31);
+  if (predict) {
+    clear_keys(L.lt_keys, (size_t)P.seps.world << rlog2, gtid, gsz);
+    phase_spmv_loss(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, threadIdx.x & 31, false);
     PSB_TRACE(L, gtid, 3);
   }
 }
@@ -952,7 +956,7 @@ __global__ void k_localize(FtrlPeers P, Minibatch M, LocalScratch L) {
 __global__ void k_spmv_loss(FtrlPeers P, Minibatch M, LocalScratch L) {
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gtid == 0) L.stats[1] += (double)M.rows;
-  phase_spmv_loss(M, L, Refs(P, P.region_log2), gtid >> 5, ((size_t)gridDim.x * blockDim.x) >> 5, threadIdx.x & 31);
+  phase_spmv_loss(M, L, Refs(P, P.region_log2), gtid >> 5, ((size_t)gridDim.x * blockDim.x) >> 5, threadIdx.x & 31, true);
 }
 __global__ void k_grad(FtrlPeers P, Minibatch M, LocalScratch L) {
   const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1050,9 +1054,8 @@ __global__ void k_apply(ShardSlot* tab, uint64_t mask, uint32_t shift, int max_p
   }
   apply_flush(acc, stats);
 }
-// empties the key table as far as the last pull used it
-__global__ void k_clear_local(LocalScratch L, int world) {
-  clear_keys(L.lt_keys, (size_t)world << L.region[kRegionNow], (size_t)blockIdx.x * blockDim.x + threadIdx.x,
+__global__ void k_clear_local(LocalScratch L) {
+  clear_keys(L.lt_keys, L.lt_slots, (size_t)blockIdx.x * blockDim.x + threadIdx.x,
              (size_t)gridDim.x * blockDim.x);
 }
 // dump the non-zero weights of a shard: out_keys/out_w sized by capacity, *count receives the number
@@ -1148,10 +1151,10 @@ static int launch_pull(const FtrlPeers* P, const Minibatch* M, const LocalScratc
   return (int)cudaLaunchCooperativeKernel((void*)ftrl_pull_kernel, dim3(grid), dim3(256), args, 0, stream);
 }
 
-// A prediction: X·w with the weights as they are, no key is created.
+// A prediction: X·w with the weights as they are; no key is created, no statistic changes.
 int psb_ftrl_pull_spmv(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, uint32_t seq, cudaStream_t stream) {
   if (L->lt_w == nullptr || L->lt_acc == nullptr || P->in_slot == nullptr || L->region == nullptr) return (int)cudaErrorInvalidValue;
-  return launch_pull(P, M, L, seq, kPullRows, stream);
+  return launch_pull(P, M, L, seq, kPullPredict, stream);
 }
 
 // Non-zeros from which on a step takes two launches: the pull gains more from its own 8 blocks per SM than the second
@@ -1228,8 +1231,8 @@ int psb_ftrl_apply(void* tab, uint64_t mask, uint32_t shift, int max_probe, cons
   k_apply<<<flat_grid(n), 256, 0, s>>>((ShardSlot*)tab, mask, shift, max_probe, rk, rg, rc, n, *h, stats, status);
   return (int)cudaGetLastError();
 }
-int psb_ftrl_clear_local(const LocalScratch* L, int world, cudaStream_t s) {
-  k_clear_local<<<flat_grid(L->lt_slots), 256, 0, s>>>(*L, world);
+int psb_ftrl_clear_local(const LocalScratch* L, cudaStream_t s) {
+  k_clear_local<<<flat_grid(L->lt_slots), 256, 0, s>>>(*L);
   return (int)cudaGetLastError();
 }
 int psb_ftrl_dump_nonzero(const void* tab, uint64_t mask, uint64_t* out_keys, float* out_w,

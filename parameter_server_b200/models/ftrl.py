@@ -294,20 +294,18 @@ class FTRLEngine:
         """X·w for a minibatch with the current model (collective: every rank calls it between steps).
         Creates no entries in the model."""
         M, s = self._mb(mb), N.stream_ptr()
-        saved = self.stats.clone()
         if self.impl == "nccl":
+            saved = self.stats.clone()
             self.group.barrier()   # every owner's last apply kernel has finished
             self._pull_nccl(M)
+            N.check(self._lib.psb_ftrl_clear_local(C.byref(self._L), s), "clear_local")
+            self.stats.copy_(saved)
         else:
             self.pull_seq += 1
-            N.check(self._lib.psb_ftrl_pull_spmv(C.byref(self._P), C.byref(M), C.byref(self._L), C.c_uint32(self.pull_seq),
-                                                 s), "ftrl_pull_spmv")
-            self.kernel_launches += 1
-        N.check(self._lib.psb_ftrl_clear_local(C.byref(self._L), self.group.world, s), "clear_local")
+            N.check(self._lib.psb_ftrl_pull_spmv(C.byref(self._P), C.byref(M), C.byref(self._L), C.c_uint32(self.pull_seq), s),
+                    "ftrl_pull_spmv")
         self.kernel_launches += 1
-        out = self.xw[: mb.rows].clone()
-        self.stats.copy_(saved)
-        return out
+        return self.xw[: mb.rows].clone()
 
     # ------------------------------------------------------- NCCL-only baseline
     def _step_nccl(self, mb: DeviceMinibatch) -> None:

@@ -136,7 +136,9 @@ def test_minibatches_of_changing_size_and_one_without_repeated_keys(rule):
         eng.check_status()
         used.append(int(eng.region[0].item()))
         ref.step([(off.cpu().numpy(), keys.cpu().numpy().view(np.uint64), y.cpu().numpy().astype(np.float64))])
+        before = eng.stats.clone()
         xw = eng.predict(DeviceMinibatch(*small)).cpu().numpy()
+        assert torch.equal(eng.stats, before)
         rxw = ref.worker_gradient(small[0].cpu().numpy(), small[1].cpu().numpy().view(np.uint64), small[2].cpu().numpy().astype(np.float64))[5]
         np.testing.assert_allclose(xw, rxw, rtol=2e-3, atol=2e-4)
     assert used[1] < used[0] < used[4] <= eng.region_log2 and used[5] == used[4], used
