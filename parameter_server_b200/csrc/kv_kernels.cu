@@ -47,7 +47,7 @@ __device__ __forceinline__ int64_t warp_lower_bound(const uint64_t* keys, int64_
 // owners' memory between those bounds, a tile that is not ordered without them.
 // Bound by the dependent loads of a search, not by bytes.  Ordered queries among twice as many keys, one bisection
 // per key -> this: 3 x 10^6 queries 101 -> 63 us, 10^6 42 -> 32 us, 3 x 10^5 29 -> 22 us.
-constexpr int kResolveThreads = 256, kResolveStage = 4096;
+constexpr int kResolveThreads = 256, kResolveStage = 3072;   // 24 KB: eight blocks per SM
 
 template <int kPer>     // queries per thread
 __global__ void __launch_bounds__(kResolveThreads)

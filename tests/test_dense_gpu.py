@@ -145,3 +145,25 @@ def test_gather_minibatch(rows, cols, b):
         xb, xbt, yb = dense.gather_minibatch(x, y, sel, want_t)
         assert torch.equal(xb, x[sel]) and torch.equal(yb, y[sel])
         assert torch.equal(xbt, x[sel].T) if want_t else xbt is None
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 5), (64, 64), (65, 130), (1000, 4), (2048, 512), (1023, 1026), (4, 300_000)])
+def test_transpose_sizes(rows, cols):
+    from parameter_server_b200.ops import dense
+
+    x = torch.randn(rows, cols, device="cuda")
+    assert torch.equal(dense.transpose(x), x.T)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 1023, 400_001])
+@pytest.mark.parametrize("adagrad", [False, True])
+def test_sgd_update_is_the_same_for_any_alignment(n, adagrad):
+    from parameter_server_b200.ops import dense
+
+    w, g, h = torch.randn(3, n + 1, device="cuda").abs().unbind(0)
+    out = []
+    for at in (0, 1):                      # 16-byte aligned, then not
+        bufs = [torch.zeros(n + 1, device="cuda")[at: at + n].copy_(t[:n]) for t in (w, g, h)]
+        dense.sgd_update(bufs[0], bufs[1], bufs[2] if adagrad else None, 0.1, 1.0, 4)
+        out.append((bufs[0].clone(), bufs[2].clone()))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
