@@ -6,10 +6,10 @@ Key sets of n uint64 keys (Zipf(1.1) over a 2^32 key space, de-duplicated) with 
   * pull  — one kernel gathering rows from the owners over NVLink (``DeviceKVVector.pull``)
   * push  — one kernel reducing rows into the owners with ``red.add`` (``DeviceKVVector.push``)
   * the same two operations with ``all_to_all_single`` + local gather / scatter-add kernels
-and, with ``--fused``, the two fused FTRL kernels on a minibatch whose n non-zeros are n distinct keys
-(32 per row, value length 1): pull + SpMV (``psb_ftrl_pull_spmv``) and push + FTRL update
-(``psb_ftrl_push_update``), each timed alone with CUDA events, against the NCCL-only engine's pull and
-push of the same minibatch.  It reports GB/s of payload per GPU and the fraction of the NVLink roofline
+and, with ``--fused``, the fused FTRL step on a minibatch whose n non-zeros are n distinct keys (32 per
+row, value length 1): its pull (de-duplication, lookup, weights back) and its rows and push (X·w, gradient,
+FTRL update), told apart by the marks inside the kernels, against the NCCL-only engine's pull and push of
+the same minibatch.  It reports GB/s of payload per GPU and the fraction of the NVLink roofline
 (bytes that must cross NVLink / 770 GB/s measured peer-copy bandwidth per direction per GPU); for the
 fused kernels the payload is 12 bytes per key for the pull (key out, weight back) and 4 bytes for the
 push (gradient), and small key sets are reported as latency.
