@@ -933,7 +933,7 @@ darlin_pass_kernel(DarlinWorker Wk, DarlinPeers P, DarlinServer S, DarlinSched Q
 // Bound by those round trips and the barriers, not by bandwidth.  One pass on B200, darlin_pass_kernel -> this one:
 // 20,242 rows x 75 non-zeros, 300 blocks (5 k non-zeros each): 3.01 -> 1.08 ms (cluster); 677,399 rows, 300 blocks
 // (169 k each): 5.20 -> 2.75 ms; 100,000 rows x 120, 64 wide blocks in groups of 9 (1.7 M each): 0.87 -> 0.38 ms.
-constexpr int kSoloThreads = 1024;
+constexpr int kSoloThreads = 1024;      // most threads of a block
 constexpr int kSoloItems = 2;
 
 struct SoloMeta {
@@ -1419,10 +1419,18 @@ using namespace psb;
 namespace {
 int g_darlin_grid[16] = {0};
 
-// Groups of blocks with at most this many non-zeros run in one cluster of 16 blocks of 1024 threads.  Time per group,
-// cluster / whole GPU: 5 k non-zeros 3.6 / 4.3 us, 10 k 4.3 / 4.6, 20 k 5.7 / 5.2, 40 k 7.9 / 5.5, 169 k 27 / 9.2.
-// (A cluster of 8: 4.1 us at 5 k.)
-constexpr int64_t kSoloClusterNnz = 14336;
+// The form of the pass by the non-zeros of a group: one cluster of 16 thread blocks or the whole GPU, and 512 or 1024
+// threads per block (fewer warps pass a barrier sooner, more keep more loads in flight).  Time per group in us on B200:
+//   non-zeros   cluster 512 / 1024   whole GPU 512 / 1024
+//       2.5 k        3.0 / 3.2              3.8 / 4.1
+//       5 k          3.6 / 3.6              4.1 / 4.3
+//      10 k          4.6 / 4.3              4.4 / 4.6
+//      20 k          6.7 / 5.8              4.9 / 5.2
+//      40 k         10.3 / 7.9              5.4 / 5.5
+//      80 k           19 / 13               6.4 / 6.4
+//     169 k           42 / 27               9.8 / 9.1
+// (A cluster of 8 x 1024: 4.1 us at 5 k.)
+constexpr int64_t kSoloClusterNnz = 10240, kSoloClusterWideNnz = 6144, kSoloWideNnz = 65536;
 
 struct SoloPlan { int sms = 0, cluster = 0; };
 
@@ -1466,12 +1474,13 @@ int solo_launch(const DarlinWorker& Wk, const DarlinPeers& P, const DarlinServer
   const void* gr = w.vals != nullptr ? (const void*)darlin_solo_kernel<false, true> : (const void*)darlin_solo_kernel<false, false>;
   const SoloPlan plan = solo_plan(cl, w.vals != nullptr);
   const bool cluster = plan.cluster > 0 && (q.variant == 2 || (q.variant == 0 && q.group_nnz <= kSoloClusterNnz));
-  if (!cluster) return (int)cudaLaunchCooperativeKernel(gr, dim3((unsigned)plan.sms), dim3(kSoloThreads), args, 0, stream);
+  const unsigned threads = q.group_nnz <= (cluster ? kSoloClusterWideNnz : kSoloWideNnz) ? kSoloThreads / 2 : kSoloThreads;
+  if (!cluster) return (int)cudaLaunchCooperativeKernel(gr, dim3((unsigned)plan.sms), dim3(threads), args, 0, stream);
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute a{};
   a.id = cudaLaunchAttributeClusterDimension;
   a.val.clusterDim.x = (unsigned)plan.cluster; a.val.clusterDim.y = a.val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)plan.cluster); cfg.blockDim = dim3(kSoloThreads);
+  cfg.gridDim = dim3((unsigned)plan.cluster); cfg.blockDim = dim3(threads);
   cfg.stream = stream; cfg.attrs = &a; cfg.numAttrs = 1;
   return (int)cudaLaunchKernelExC(&cfg, cl, args);
 }
