@@ -931,7 +931,7 @@ darlin_pass_kernel(DarlinWorker Wk, DarlinPeers P, DarlinServer S, DarlinSched Q
 //   * kCluster: when a group has so few non-zeros that one thread-block cluster covers them, the whole pass
 //     runs in ONE cluster and the barriers are the hardware's cluster barrier.
 // Bound by those round trips and the barriers, not by bandwidth.  One pass on B200, darlin_pass_kernel -> this one:
-// 20,242 rows x 75 non-zeros, 300 blocks (5 k non-zeros each): 3.01 -> 1.08 ms (cluster); 677,399 rows, 300 blocks
+// 20,242 rows x 75 non-zeros, 300 blocks (5 k non-zeros each): 3.01 -> 1.07 ms (cluster); 677,399 rows, 300 blocks
 // (169 k each): 5.20 -> 2.75 ms; 100,000 rows x 120, 64 wide blocks in groups of 9 (1.7 M each): 0.87 -> 0.38 ms.
 constexpr int kSoloThreads = 1024;      // most threads of a block
 constexpr int kSoloItems = 2;
