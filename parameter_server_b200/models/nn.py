@@ -131,7 +131,7 @@ class DataLayer(Layer):
         else:
             b -= b % 4        # GEMM operand strides are multiples of 4 floats
             sel = torch.randperm(n, generator=self.gen)[:b].to(self.net.device)
-            if self.X.is_cuda and self.y.is_contiguous() and b <= 32 * 65535:
+            if dense.can_gather_minibatch(self.X, self.y, b):
                 xb, xbt, yb = dense.gather_minibatch(self.X, self.y, sel, self.net.training and self.outputs[0].read_by_dense)
                 self.outputs[0].transposed = None if xbt is None else (xb, xb._version, xbt)
             else:

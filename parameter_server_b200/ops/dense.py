@@ -80,10 +80,16 @@ def act_backward_t(g: torch.Tensor, y: torch.Tensor, act: str, want_z: bool = Tr
     return z, zt
 
 
+def can_gather_minibatch(x: torch.Tensor, y: torch.Tensor, b: int) -> bool:
+    """The data that :func:`gather_minibatch` takes: one label per row (labels of several columns are indexed)."""
+    return (x.is_cuda and x.device == y.device and x.dtype == y.dtype == torch.float32 and x.dim() == 2 and y.shape == x.shape[:1]
+            and x.shape[1] > 0 and x.is_contiguous() and y.is_contiguous() and 0 < b <= 32 * 65535)
+
+
 def gather_minibatch(x: torch.Tensor, y: torch.Tensor, sel: torch.Tensor, want_t: bool):
     """(``x[sel]``, its transpose or None, ``y[sel]``) for contiguous float32 ``x`` [n, cols], ``y`` [n] and device
     int64 row numbers ``sel`` (all inside x), in one launch."""
-    assert x.is_contiguous() and y.is_contiguous() and sel.is_contiguous() and x.dtype == y.dtype == torch.float32 and sel.dtype == torch.int64
+    assert can_gather_minibatch(x, y, sel.numel()) and sel.device == x.device and sel.is_contiguous() and sel.dtype == torch.int64
     b, cols = sel.numel(), x.shape[1]
     xb = torch.empty((b, cols), dtype=torch.float32, device=x.device)
     yb = torch.empty(b, dtype=torch.float32, device=x.device)

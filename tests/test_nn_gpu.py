@@ -152,3 +152,26 @@ def test_sparse_net_trains():
     sol.train.layer("data").set_sparse_data(off, idx, vals, y, 300)
     hist = sol.run(verbose=False)
     assert sum(h["loss"] for h in hist[-10:]) < 0.8 * sum(h["loss"] for h in hist[:10])
+
+
+@pytest.mark.parametrize("columns", [None, 1, 3])
+def test_minibatch_takes_the_labels_of_its_rows(columns):
+    """Labels are one per row, or a column per output unit: a minibatch holds those of its rows, in their shape."""
+    from parameter_server_b200 import config as cfg
+    from parameter_server_b200.models.nn import SGDSolver
+    from parameter_server_b200.parallel.peer import PeerGroup
+
+    conf = cfg.parse_app_config((NET % (40, "RELU", "RELU", "NORMAL", 0.1, 1, 0)).replace('"s1"', '"s"').replace("size: 4", f"size: {columns or 1}"))
+    sol = SGDSolver(conf.neural_network, PeerGroup.single(torch.device("cuda", 0)))
+    X, _ = _data(200, 8, 6)
+    X[:, 0] = torch.arange(200)                   # tells the rows of a minibatch
+    y = torch.where(torch.rand(200 * (columns or 1), generator=torch.Generator().manual_seed(1)) < 0.5, 1.0, -1.0)
+    y = y if columns is None else y.reshape(200, columns)
+    sol.train.layer("data").set_data(X, y, normalize=False)
+    sol.train.forward()
+    xb, yb = sol.train.edge("x").value, sol.train.edge("y").value
+    rows = xb[:, 0].long().cpu()
+    assert torch.equal(xb.cpu(), X[rows]) and torch.equal(yb.cpu(), y[rows])
+    s = sol.train.edge("s").value
+    want = torch.nn.functional.softplus(-s.reshape(-1).double() * yb.reshape(-1)).sum().item()
+    assert sol.train.layer("loss").loss.item() == pytest.approx(want, rel=1e-5)
