@@ -141,7 +141,12 @@ def columns_from_rows(offsets: torch.Tensor, keys: torch.Tensor, vals: Optional[
     """CSR rows over uint64 keys → column-major storage over the unique keys, with one stable sort of the non-zeros:
     (unique keys in unsigned order, col_ptr int64, row_idx int32, vals, column of every non-zero int32 or None).
     ``Localizer::countUniqIndex`` + ``remapIndex`` + ``SparseMatrix::alterStorage``; the rows of a column ascend."""
-    lib, n, dev, rows = _lib(), keys.numel(), keys.device, offsets.numel() - 1
+    n, dev, rows = keys.numel(), keys.device, offsets.numel() - 1
+    if offsets.device != dev or (vals is not None and vals.device != dev):
+        raise ValueError(f"row offsets and values must be where the keys are ({dev})")
+    if vals is not None and vals.numel() != n:
+        raise ValueError(f"{vals.numel()} values for {n} non-zeros")
+    lib = _lib()
     keys, offsets = keys.contiguous(), offsets.to(torch.int64).contiguous()
     if n == 0 or n >= 1 << 32 or (vals is not None and vals.dtype != torch.float32):   # positions travel as 32-bit payloads
         lkeys, _ = count_unique(keys)

@@ -127,3 +127,19 @@ def test_bin_matrix_roundtrip(tmp_path):
     assert sub["rows"] == 2 and sub["offset"].tolist() == [0, 0, 3] and sub["index"].tolist() == [0, 2, 3]
     assert H.write_bin_matrix(name + "b", False, 3, 5, off, idx)
     assert H.read_bin_matrix(name + "b")["binary"] and H.read_bin_matrix(str(tmp_path / "nope")) is None
+
+
+def test_columns_from_rows_refuses_values_and_offsets_that_do_not_belong_to_the_keys():
+    """Checked before anything is launched: a kernel would read a host address or past the values."""
+    import torch
+
+    from parameter_server_b200.ops import sparse
+
+    keys = torch.zeros(4, dtype=torch.int64, device="meta")      # stands for the device
+    off = torch.tensor([0, 1, 4])
+    with pytest.raises(ValueError, match="where the keys are"):
+        sparse.columns_from_rows(off, keys, None)
+    with pytest.raises(ValueError, match="where the keys are"):
+        sparse.columns_from_rows(off.to("meta"), keys, torch.ones(4))
+    with pytest.raises(ValueError, match="3 values for 4"):
+        sparse.columns_from_rows(off.to("meta"), keys, torch.ones(3, device="meta"))
