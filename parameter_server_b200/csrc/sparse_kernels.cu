@@ -177,13 +177,15 @@ __global__ void k_counts_from_starts(const unsigned long long* __restrict__ usta
 // 0.15 M over 20,000 2.03 -> 1.47.
 constexpr int kColThreads = 256, kColItems = 8, kColTile = kColThreads * kColItems;
 
-// row of every non-zero, one warp per row
-__global__ void k_row_ids(const int64_t* __restrict__ off, int64_t rows, size_t n, uint32_t* __restrict__ row) {
+// row of every non-zero, one warp per row; a row is walked inside [0, n), whatever its offsets say (the caller checks
+// them afterwards, and offsets far apart would otherwise be a walk without end)
+__global__ void k_row_ids(const int64_t* __restrict__ off, int64_t rows, int64_t n, uint32_t* __restrict__ row) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw)
-    for (int64_t i = off[r] - off[0] + lane; i < off[r + 1] - off[0]; i += 32)
-      if ((size_t)i < n) row[i] = (uint32_t)r;
+  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
+    const int64_t b = off[r] - off[0], e = off[r + 1] - off[0], end = e < n ? e : n;
+    for (int64_t i = (b > 0 ? b : 0) + lane; i < end; i += 32) row[i] = (uint32_t)r;
+  }
 }
 __global__ void k_iota_u32(uint32_t* __restrict__ out, size_t n) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) out[i] = (uint32_t)i;
@@ -420,7 +422,7 @@ int psb_counts_from_starts(const unsigned long long* ustart, size_t nu, size_t n
   return (int)cudaGetLastError();
 }
 int psb_row_ids(const int64_t* off, int64_t rows, size_t n, uint32_t* row, cudaStream_t s) {
-  k_row_ids<<<g1((size_t)rows * 32), 256, 0, s>>>(off, rows, n, row);
+  k_row_ids<<<g1((size_t)rows * 32), 256, 0, s>>>(off, rows, (int64_t)n, row);
   return (int)cudaGetLastError();
 }
 int psb_iota_u32(uint32_t* out, size_t n, cudaStream_t s) {

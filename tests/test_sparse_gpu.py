@@ -143,3 +143,13 @@ def test_columns_from_rows(rows, per_row, keys, valued):
     assert torch.equal(sparse.columns_from_rows(d(off + 9), d(key), None)[2], row_idx)
     with pytest.raises((ValueError, RuntimeError, IndexError)):      # rows that do not describe the non-zeros
         sparse.columns_from_rows(d(np.concatenate([off[:-1], [n + 3]])), d(key), None)
+
+
+def test_columns_from_rows_refuses_offsets_that_go_astray():
+    """Offsets far outside the non-zeros are an error of the host, found after a walk that stays inside them."""
+    from parameter_server_b200.ops import sparse
+
+    keys = torch.arange(100, device="cuda")
+    for off in ([0, 1 << 62, 100], [0, -(1 << 62), 100], [0, 50, 1 << 61], [7, 1 << 62, -(1 << 62), 107]):
+        with pytest.raises(ValueError):
+            sparse.columns_from_rows(torch.tensor(off, device="cuda"), keys, None)
