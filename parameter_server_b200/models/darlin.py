@@ -596,6 +596,12 @@ class DarlinSolver:
                 return self.launch_pass(order, first=first)
             finally:
                 self.cfg.max_block_delay = saved
+        if self.cfg.max_block_delay > 0 and self.group.world == 1 and self.impl == "fused" and not self.out_of_core:
+            cut = repeat_in_group(order, self.cfg.max_block_delay + 1)
+            while cut:       # two threads would step that block's columns
+                self.launch_pass(order[:cut], first=first)
+                order, first = order[cut:], False
+                cut = repeat_in_group(order, self.cfg.max_block_delay + 1)
         order_t = torch.as_tensor(order, dtype=torch.int32).to(self.dev, non_blocking=False)
         self._order_keepalive = order_t
         if first:
@@ -799,6 +805,18 @@ class DarlinSolver:
         path = f"{file_prefix}_S{self.group.rank}"
         write_model_text(path, k, w)
         return path
+
+
+def repeat_in_group(order, group: int) -> int:
+    """Position of the first block of ``order`` that its group of ``group`` consecutive entries holds already (0: none).
+    A group that ends there is a shorter delay, which the bound allows."""
+    order = np.asarray(order)
+    if len(order) < 2 or np.bincount(order).max() < 2:
+        return 0
+    for i in range(1, len(order)):
+        if order[i] in order[i // group * group: i]:
+            return i
+    return 0
 
 
 def print_progress(it: int, p: Progress, file=sys.stderr, busy=None) -> None:

@@ -143,6 +143,30 @@ def test_block_swept_twice_in_a_row_sees_its_own_update(variant):
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-5)      # sums of the same terms in another order
 
 
+@pytest.mark.parametrize("wide", [0, 1])
+@pytest.mark.parametrize("variant", [1, 2])
+def test_block_twice_in_one_bounded_delay_group(variant, wide):
+    """A block that its group holds already ends the group: it is swept twice, and the margins are those of the weights."""
+    from parameter_server_b200.models.darlin import DarlinConfig, DarlinSolver, margins_from_weights
+    from parameter_server_b200.parallel.peer import PeerGroup
+
+    off, keys, vals, y = _problem(False)
+    got = []
+    for orders, tau in (([[0, 1, 1, 0, 0, 1]], 2), ([[0, 1], [1, 0], [0, 1]], 1)):
+        sol = DarlinSolver(PeerGroup.single(torch.device("cuda", 0)),
+                           DarlinConfig(lambda1=0.3, feature_block_ratio=0.5, seed=3, max_block_delay=tau), wide_block_cols=wide)
+        sol.pass_variant = variant
+        sol.preprocess(off, keys, vals, y)
+        for o in orders:
+            sol.launch_pass(np.asarray(o, dtype=np.int32))
+        sol.check_status()
+        want = margins_from_weights(sol.col_ptr, sol.row_idx, sol.vals, sol.y, sol.w)
+        assert torch.allclose(sol.margin, want, rtol=1e-4, atol=1e-4)
+        got.append((sol.w.clone(), sol.margin.clone(), sol.delta.clone()))
+    for a, b in zip(*got):
+        assert torch.allclose(a, b, rtol=1e-4, atol=1e-5)      # sums of the same terms in another order
+
+
 def test_tail_feature_filter_drops_rare_columns():
     """Columns whose count-min estimate is <= tail_feature_freq are removed before training; the rest of the
     run equals the oracle on the data filtered by a NumPy restatement of the same sketch."""

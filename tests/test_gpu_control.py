@@ -252,3 +252,13 @@ def test_online_job_failure_reaches_the_scheduler(tmp_path):
 def test_online_job_does_not_hang_when_a_rank_vanishes(tmp_path):
     got = _run_online("vanish", tmp_path, expect=1)
     assert got[0][0] == "error" and ("W0:" in got[0][1] or "no heartbeat" in got[0][1] or "task failed" in got[0][1]), got
+
+
+def test_repeat_in_group():
+    import numpy as np
+
+    from parameter_server_b200.models.darlin import repeat_in_group
+
+    for order, group, want in (([], 3, 0), ([2], 3, 0), ([0, 1, 2, 0], 3, 0), ([0, 1, 0, 2], 3, 2), ([5, 5], 2, 1), ([5, 5], 1, 0),
+                               ([0, 1, 2, 3, 4, 3], 3, 5), ([0, 1, 2, 1, 0], 3, 0)):
+        assert repeat_in_group(np.asarray(order, dtype=np.int32), group) == want, order
