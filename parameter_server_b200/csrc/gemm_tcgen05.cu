@@ -435,8 +435,9 @@ k_gemm_rank4(const float* __restrict__ a, const float* __restrict__ b, float* __
   for (int j = 0; j < 4; ++j)
 #pragma unroll
     for (int k = 0; k < 4; ++k) w[j][k] = n0 + j < N && k < K ? tf32_cut(b[(size_t)(n0 + j) * ldb + k]) : 0.f;
-  const int m0 = blockIdx.y * kRankRows, m1 = m0 + kRankRows < M ? m0 + kRankRows : M;
-  for (int m = m0; m < m1; ++m) {
+  // groups of kRankRows rows, gridDim.y apart (a grid has at most 65,535 of them)
+  for (int64_t g = (int64_t)blockIdx.y * kRankRows; g < M; g += (int64_t)gridDim.y * kRankRows)
+  for (int m = (int)g, m1 = M - m > kRankRows ? m + kRankRows : M; m < m1; ++m) {
     float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -686,9 +687,10 @@ int psb_gemm_tn_tf32(const float* a, const float* b, float* out, float* out_t, i
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const bool aligned = ((lda | ldb) & 3) == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
   if (variant == 3 ? K > 4 : !aligned) return (int)cudaErrorInvalidValue;
-  const dim3 rank_grid((N + 1023) / 1024, (M + kRankRows - 1) / kRankRows);
+  const unsigned row_groups = ((unsigned)M + kRankRows - 1) / kRankRows;
+  const dim3 rank_grid((N + 1023) / 1024, row_groups < 65535u ? row_groups : 65535u);
   const long tiles_d = (long)((M + kDTile - 1) / kDTile) * ((N + kDTile - 1) / kDTile);
-  if (variant == 0) variant = K <= 4 && rank_grid.y < 65536u ? 3 : tiles_d >= kPairTiles ? 2 : 1;
+  if (variant == 0) variant = K <= 4 ? 3 : tiles_d >= kPairTiles ? 2 : 1;
   if (variant == 3) {
     k_gemm_rank4<<<rank_grid, 256, 0, stream>>>(a, b, out, out_t, M, N, K, lda, ldb, ldo, act);
     return (int)cudaGetLastError();

@@ -167,3 +167,14 @@ def test_sgd_update_is_the_same_for_any_alignment(n, adagrad):
         dense.sgd_update(bufs[0], bufs[1], bufs[2] if adagrad else None, 0.1, 1.0, 4)
         out.append((bufs[0].clone(), bufs[2].clone()))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("M,K", [(1_048_560, 1), (1_048_561, 2), (1_100_003, 3), (2_200_000, 4)])
+def test_outer_product_of_more_rows_than_a_grid_has_blocks(M, K):
+    from parameter_server_b200.ops import dense
+
+    a, b = torch.randn(M, K, device="cuda"), torch.randn(8, K, device="cuda")
+    t = torch.full((8, M), float("nan"), device="cuda")
+    out = dense.gemm_tn(a, b, pad_k=True, out_t=t)
+    ref, bound = a.double() @ b.double().T, (a.double().abs() @ b.double().abs().T) / 512 + 1e-5      # TF32 operands
+    assert bool(((out.double() - ref).abs() <= bound).all()) and torch.equal(t, out.T)

@@ -175,3 +175,18 @@ def test_minibatch_takes_the_labels_of_its_rows(columns):
     s = sol.train.edge("s").value
     want = torch.nn.functional.softplus(-s.reshape(-1).double() * yb.reshape(-1)).sum().item()
     assert sol.train.layer("loss").loss.item() == pytest.approx(want, rel=1e-5)
+
+
+def test_full_batch_of_more_than_a_million_rows():
+    """One output, three inputs: the outer products of both ends of the net have a row per example."""
+    sol = _solver("RELU", "NORMAL", 1e-6, 1, batch=0)
+    X, y = _data(1_100_000, 3, 8)
+    sol.train.layer("data").set_data(X, y, normalize=False)
+    sol.train.forward()
+    sol.train.backward()
+    w1, w2 = (sol.train.layer(n).model.value.double().requires_grad_(True) for n in ("fc1", "fc2"))
+    s = (torch.relu(X.cuda().double() @ w1.T) @ w2.T).reshape(-1)
+    torch.nn.functional.softplus(-s * y.cuda()).sum().backward()
+    for name, ref in (("fc1", w1.grad), ("fc2", w2.grad)):
+        got = sol.train.layer(name).model.gradient
+        assert (got - ref).abs().max().item() < 2e-2 * ref.abs().max().item()
