@@ -716,8 +716,9 @@ int psb_gemm_tn_tf32(const float* a, const float* b, float* out, float* out_t, i
   if (M <= kThinRows) return launch_tile<kThinRows, kThinCols>(a, b, out, out_t, M, N, K, lda, ldb, ldo, act, status, stream);
   return launch_tile<kBM, kBN>(a, b, out, out_t, M, N, K, lda, ldb, ldo, act, status, stream);
 }
+// An empty matrix is refused here and in psb_act_backward_t: it is a minibatch without rows, whose gradients nothing would write.
 int psb_transpose(const float* in, float* out, int rows, int cols, cudaStream_t s) {
-  if (rows <= 0 || cols <= 0) return 0;
+  if (rows <= 0 || cols <= 0) return (int)cudaErrorInvalidConfiguration;
   const dim3 grid((cols + kActTile - 1) / kActTile, (rows + kActTile - 1) / kActTile);
   if (grid.y > 65535u) return (int)cudaErrorInvalidValue;
   // 32 x 32 tiles of single floats / 64 x 64 tiles of float4 on B200, L2 flushed: 256x64 6.2 / 8.2 us (few blocks, each with a
@@ -747,7 +748,7 @@ int psb_act_backward(const float* g, const float* y, float* z, size_t n, int act
 }
 // z (may be null) and its transpose zt [cols, rows]
 int psb_act_backward_t(const float* g, const float* y, float* z, float* zt, int rows, int cols, int act, cudaStream_t s) {
-  if (rows <= 0 || cols <= 0) return 0;
+  if (rows <= 0 || cols <= 0) return (int)cudaErrorInvalidConfiguration;
   const uintptr_t all = reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(zt);
   const dim3 grid((cols + kActTile - 1) / kActTile, (rows + kActTile - 1) / kActTile);
   if (grid.y > 65535u) return (int)cudaErrorInvalidValue;

@@ -144,7 +144,7 @@ class DataLayer(Layer):
 
 def _transposed(x: torch.Tensor) -> torch.Tensor:
     """``xᵀ``, contiguous, to be read only: a single row or column is laid out like its transpose."""
-    return x.reshape(x.shape[1], x.shape[0]) if 1 in x.shape and x.is_contiguous() else dense.transpose(x)
+    return x.reshape(x.shape[1], x.shape[0]) if 1 in x.shape and x.numel() and x.is_contiguous() else dense.transpose(x)
 
 
 class FullyConnectedLayer(Layer):

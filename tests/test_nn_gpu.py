@@ -190,3 +190,13 @@ def test_full_batch_of_more_than_a_million_rows():
     for name, ref in (("fc1", w1.grad), ("fc2", w2.grad)):
         got = sol.train.layer(name).model.gradient
         assert (got - ref).abs().max().item() < 2e-2 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("act", ["RELU", "IDENTITY"])
+def test_training_on_a_minibatch_without_rows_is_refused(act):
+    """A minibatch size is cut to a multiple of four: fewer than four rows are none, and no gradient comes of them."""
+    sol = _solver(act, "NORMAL", 0.1, 1, batch=3)
+    sol.train.layer("data").set_data(*_data(100, 8, 9), normalize=False)
+    sol.train.forward()
+    with pytest.raises(RuntimeError):
+        sol.train.backward()
