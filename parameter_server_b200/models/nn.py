@@ -143,8 +143,9 @@ class DataLayer(Layer):
 
 
 def _transposed(x: torch.Tensor) -> torch.Tensor:
-    """``xᵀ``, contiguous, to be read only: a single row or column is laid out like its transpose."""
-    return x.reshape(x.shape[1], x.shape[0]) if 1 in x.shape and x.numel() and x.is_contiguous() else dense.transpose(x)
+    """``xᵀ``, contiguous and 16-byte aligned, to be read only: a single row or column is laid out like its transpose."""
+    same = 1 in x.shape and x.numel() > 0 and x.is_contiguous() and x.data_ptr() % 16 == 0
+    return x.reshape(x.shape[1], x.shape[0]) if same else dense.transpose(x)
 
 
 class FullyConnectedLayer(Layer):
