@@ -53,7 +53,7 @@ def ops(monkeypatch):
 
     for f in (gemm_tn, act_backward_t, logistic_loss, sgd_update):
         monkeypatch.setattr(dense, f.__name__, f)
-    monkeypatch.setattr(dense, "transpose", lambda x: x.T.contiguous())
+    monkeypatch.setattr(dense, "transpose", lambda x: x.T.clone(memory_format=torch.contiguous_format))
     monkeypatch.setattr(dense, "check_status", lambda dev: None)
     return asked
 
