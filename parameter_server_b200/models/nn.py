@@ -132,8 +132,8 @@ class DataLayer(Layer):
             b -= b % 4        # GEMM operand strides are multiples of 4 floats
             sel = torch.randperm(n, generator=self.gen)[:b].to(self.net.device)
             if dense.can_gather_minibatch(self.X, self.y, b):
-                xb, xbt, yb = dense.gather_minibatch(self.X, self.y, sel, self.net.training and self.outputs[0].read_by_dense)
-                self.outputs[0].transposed = None if xbt is None else (xb, xb._version, xbt)
+                xb, xbt, yb = dense.gather_minibatch(self.X, self.y, sel, self.net.keeps_transpose(self.outputs[0], b * self.X.shape[1]))
+                self.outputs[0].keep_transpose(xb, xbt)
             else:
                 xb, yb = self.X[sel].contiguous(), self.y[sel].contiguous()
         self.outputs[0].value = xb
@@ -177,9 +177,9 @@ class FullyConnectedLayer(Layer):
         out = self.outputs[0]
         # a dense layer that reads this edge needs its transpose for the weight gradient: the GEMM writes both
         yt = torch.empty((self.out_dim, x.shape[0]), dtype=torch.float32, device=x.device) \
-            if self.net.training and out.read_by_dense else None
+            if self.net.keeps_transpose(out, x.shape[0] * self.out_dim) else None
         out.value = dense.gemm_tn(x, self.model.value, self.act, pad_k=True, out_t=yt)
-        out.transposed = None if yt is None else (out.value, out.value._version, yt)
+        out.keep_transpose(out.value, yt)
         return 0.0
 
     def backward(self) -> None:
@@ -188,8 +188,8 @@ class FullyConnectedLayer(Layer):
             z, zt = gy, _transposed(gy)
         else:
             z, zt = dense.act_backward_t(gy, y, self.act, want_z=self.inputs[0].needs_grad)
-        t, self.inputs[0].transposed = self.inputs[0].transposed, None
-        xt = t[2] if t is not None and t[0] is self.x and t[0]._version == t[1] else _transposed(self.x)
+        xt = self.inputs[0].take_transpose(self.x)
+        xt = _transposed(self.x) if xt is None else xt
         self.model.gradient = dense.gemm_tn(zt, xt, pad_k=True)                       # [out, in] = Zᵀ · X
         if self.inputs[0].needs_grad:
             wt = _transposed(self.model.value)                            # [in, out]
@@ -261,6 +261,16 @@ class Edge(Parameter):
     read_by_dense: bool = False                  # a fully connected layer has this edge as its input
     transposed: Optional[tuple] = None           # (value, its version, valueᵀ) from the layer that wrote the value
 
+    def keep_transpose(self, value: torch.Tensor, t: Optional[torch.Tensor]) -> None:
+        """``t`` is ``valueᵀ`` (None: it is not at hand) until the value is written to.  A tensor of inference mode does
+        not tell when it was written to, and its transpose is not kept."""
+        self.transposed = None if t is None or value.is_inference() else (value, value._version, t)
+
+    def take_transpose(self, value: torch.Tensor) -> Optional[torch.Tensor]:
+        """The kept transpose of ``value`` if it still is that; it is not kept any longer."""
+        t, self.transposed = self.transposed, None
+        return t[2] if t is not None and t[0] is value and value._version == t[1] else None
+
 
 class Net:
     """Layers wired by edge names, executed in the listed (topological) order."""
@@ -286,6 +296,11 @@ class Net:
         if name not in self.edges:
             self.edges[name] = Edge(name)
         return self.edges[name]
+
+    def keeps_transpose(self, edge: Edge, numel: int) -> bool:
+        """Whether the layer that writes ``numel`` elements to ``edge`` writes their transpose too, for the weight
+        gradient of the dense layer that reads it."""
+        return self.training and edge.read_by_dense and not torch.is_inference_mode_enabled()
 
     def layer(self, name: str) -> Layer:
         return next(l for l in self.layers if l.name == name)

@@ -94,3 +94,20 @@ def test_one_feature_from_a_view_of_any_alignment(ops, offset):
     sol.train.forward()
     sol.train.backward()
     _check_gradients(sol, X, y)
+
+
+def test_training_inside_inference_mode(ops):
+    """Gradients are the layers' own, so a net trains where autograd is off; such tensors have no version counter."""
+    sol, X, y = _net()
+    with torch.inference_mode():
+        sol.train.layer("data").set_data(X.clone(), y.clone(), normalize=False)
+        sol.train.forward()
+        sol.train.backward()
+        got = [sol.train.layer(n).model.gradient.clone() for n in ("fc1", "fc2", "fc3")]
+        loss = sol.step(0)
+    sol2, _, _ = _net()
+    sol2.train.forward()
+    sol2.train.backward()
+    for n, g in zip(("fc1", "fc2", "fc3"), got):
+        torch.testing.assert_close(g, sol2.train.layer(n).model.gradient)
+    assert loss > 0
