@@ -111,3 +111,21 @@ def test_training_inside_inference_mode(ops):
     for n, g in zip(("fc1", "fc2", "fc3"), got):
         torch.testing.assert_close(g, sol2.train.layer(n).model.gradient)
     assert loss > 0
+
+
+def test_kept_transposes_are_bounded(ops, monkeypatch):
+    """Transposes wait for the backward pass up to a bound; what is beyond it is transposed when it is needed."""
+    from parameter_server_b200.models import nn
+
+    monkeypatch.setattr(nn, "KEPT_TRANSPOSE_BYTES", 16 * 8 * 4 + 100)
+    sol, X, y = _net(sizes=(12, 8))
+    for _ in range(2):                       # the bound holds for a step, not for the life of the net
+        ops.clear()
+        sol.train.forward()
+        assert sum(t[2].numel() * 4 for t in (e.transposed for e in sol.train.edges.values()) if t is not None) <= 16 * 8 * 4 + 100
+        assert ops == [16 * 8 * 4]           # the first hidden layer's transpose is too large, the second's fits
+        sol.train.backward()
+        _check_gradients(sol, X, y)
+    sol.train.forward()                      # ... and holds when no backward pass came between
+    sol.train.forward()
+    assert ops == [16 * 8 * 4] * 3
