@@ -28,6 +28,12 @@ def check_status(dev) -> None:
         raise RuntimeError(f"GEMM kernel gave up waiting (code {st[0]}, tile {st[1]},{st[2] - 100})")
 
 
+def _written(t: torch.Tensor) -> None:
+    """A kernel wrote to a tensor of the caller's: its version counter says so, as after PyTorch's in-place operators."""
+    if not t.is_inference():
+        torch.autograd.graph.increment_version(t)
+
+
 def gemm_tn(a: torch.Tensor, b: torch.Tensor, act: str = "IDENTITY", out: Optional[torch.Tensor] = None,
             pad_k: bool = False, out_t: Optional[torch.Tensor] = None, variant: int = 0) -> torch.Tensor:
     """``act(a @ b.T)`` for row-major fp32 ``a`` [M,K] and ``b`` [N,K] on the tcgen05 tensor cores (TF32).  ``out_t``
@@ -47,6 +53,8 @@ def gemm_tn(a: torch.Tensor, b: torch.Tensor, act: str = "IDENTITY", out: Option
         K = kp
     if out is None:
         out = torch.empty((M, Nn), dtype=torch.float32, device=a.device)
+    else:
+        _written(out)
     if out_t is not None:
         assert out_t.shape == (Nn, M) and out_t.is_contiguous() and out_t.dtype == torch.float32
     rc = N.lib().psb_gemm_tn_tf32(N.ptr(a), N.ptr(b), N.ptr(out), N.ptr(out_t), M, Nn, K, a.stride(0), b.stride(0), out.stride(0),
@@ -115,6 +123,7 @@ def sgd_update(w: torch.Tensor, g: torch.Tensor, h: Optional[torch.Tensor], alph
 def col_normalize(x: torch.Tensor) -> None:
     assert x.is_contiguous() and x.dim() == 2
     N.check(N.lib().psb_col_normalize(N.ptr(x), x.shape[0], x.shape[1], N.stream_ptr()), "col_normalize")
+    _written(x)
 
 
 def sparse_fc_forward(off: torch.Tensor, idx: torch.Tensor, vals: Optional[torch.Tensor], w: torch.Tensor, act: str = "IDENTITY") -> torch.Tensor:

@@ -200,3 +200,24 @@ def test_training_on_a_minibatch_without_rows_is_refused(act):
     sol.train.forward()
     with pytest.raises(RuntimeError):
         sol.train.backward()
+
+
+@pytest.mark.parametrize("how", ["col_normalize", "gemm_tn", "torch"])
+def test_activation_written_to_between_forward_and_backward(how):
+    """The weight gradient is that of the activation as it is when the backward pass reads it."""
+    from parameter_server_b200.ops import dense
+
+    sol = _solver("RELU", "NORMAL", 0.1, 1, batch=0)
+    sol.train.layer("data").set_data(*_data(512, 32, 10), normalize=False)
+    sol.train.forward()
+    h = sol.train.edge("h").value
+    if how == "col_normalize":
+        dense.col_normalize(h)
+    elif how == "gemm_tn":
+        dense.gemm_tn(torch.randn(512, 32, device="cuda"), torch.randn(64, 32, device="cuda"), out=h)
+    else:
+        h.mul_(2.0)
+    sol.train.backward()
+    want = sol.train.edge("s").gradient.double().T @ h.double()
+    got = sol.train.layer("fc2").model.gradient
+    assert (got - want).abs().max().item() < 2e-2 * want.abs().max().item()
