@@ -81,6 +81,7 @@ def act_backward(g: torch.Tensor, y: torch.Tensor, act: str) -> torch.Tensor:
 def act_backward_t(g: torch.Tensor, y: torch.Tensor, act: str, want_z: bool = True):
     """(``g ∘ act'(y)`` or None, its transpose) of two contiguous [rows, cols] matrices in one pass over them."""
     assert g.is_contiguous() and y.is_contiguous() and g.shape == y.shape and g.dim() == 2
+    assert g.is_cuda and g.device == y.device and g.dtype == y.dtype == torch.float32
     z = torch.empty_like(g) if want_z else None
     zt = torch.empty((g.shape[1], g.shape[0]), dtype=torch.float32, device=g.device)
     N.check(N.lib().psb_act_backward_t(N.ptr(g), N.ptr(y), N.ptr(z), N.ptr(zt), g.shape[0], g.shape[1], ACT[act], N.stream_ptr()),

@@ -129,3 +129,11 @@ def test_kept_transposes_are_bounded(ops, monkeypatch):
     sol.train.forward()                      # ... and holds when no backward pass came between
     sol.train.forward()
     assert ops == [16 * 8 * 4] * 3
+
+
+def test_slope_and_transpose_take_float32_on_the_device_only():
+    """As the transpose that they replace did; the kernel would read other data as floats."""
+    g = torch.ones(4, 4)
+    for a, b in ((g.double(), g.double()), (g, g.double()), (g.half(), g.half()), (g, g)):
+        with pytest.raises(AssertionError):
+            dense.act_backward_t(a, b, "RELU")
