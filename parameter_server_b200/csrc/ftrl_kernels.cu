@@ -688,7 +688,9 @@ __device__ __forceinline__ SlotWords load_slot(const ShardSlot* p) {
 __device__ __forceinline__ void store_slot(ShardSlot* p, const SlotWords& v) {
   asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(v.key), "l"(v.wz), "l"(v.pn), "l"(v.reserved) : "memory");
 }
-// The key of a slot is written once, before any update of it, so storing it again changes nothing.
+// The key of a slot is written once, before any update of it, so storing it again changes nothing.  A caller that may
+// have entered the key just now stores the key it has: a 32-byte load need not see this thread's own 8-byte
+// compare-and-swap, since the memory model orders accesses of the same size only.
 __device__ __forceinline__ void apply_slot(ShardSlot* tab, uint32_t slot, SlotWords v, float g, uint32_t dpos, uint32_t dneg,
                                            const FtrlHyper& h, ApplyAcc& acc) {
   ShardState e{__uint_as_float((uint32_t)v.wz), __uint_as_float((uint32_t)(v.wz >> 32)), (uint32_t)v.pn, (uint32_t)(v.pn >> 32)};
@@ -825,7 +827,9 @@ __device__ __forceinline__ void phase_apply_filtered(cg::grid_group& grid, const
         slot = shard_find_or_insert(P.tab, P.tab_mask, P.tab_shift, key, P.max_probe, &w, &acc.dins);
         if (slot == kAbsent) { set_status(L.status, kShardTableFull, 0, 0); continue; }
       }
-      apply_slot(P.tab, slot, load_slot(P.tab + slot), g, dpos, dneg, H, acc);
+      SlotWords v = load_slot(P.tab + slot);
+      v.key = key;
+      apply_slot(P.tab, slot, v, g, dpos, dneg, H, acc);
     }
     grid.sync();
   }
@@ -1050,7 +1054,9 @@ __global__ void k_apply(ShardSlot* tab, uint64_t mask, uint32_t shift, int max_p
     const uint32_t slot = shard_find_or_insert(tab, mask, shift, key, max_probe, &w, &acc.dins);
     if (slot == kAbsent) { set_status(status, kShardTableFull, 0, 0); continue; }
     const uint64_t c = __ldcg(rc + i);
-    apply_slot(tab, slot, load_slot(tab + slot), __ldcg(rg + i), (uint32_t)(c >> 32), (uint32_t)c, h, acc);
+    SlotWords v = load_slot(tab + slot);
+    v.key = key;
+    apply_slot(tab, slot, v, __ldcg(rg + i), (uint32_t)(c >> 32), (uint32_t)c, h, acc);
   }
   apply_flush(acc, stats);
 }

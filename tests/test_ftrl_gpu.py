@@ -181,6 +181,28 @@ def test_rows_of_all_lengths(rule, valued, launches, log2):
     np.testing.assert_allclose(w, rw, rtol=2e-3, atol=2e-5)
 
 
+@pytest.mark.parametrize("impl", ["fused", "nccl"])
+def test_keys_entered_by_the_update_itself_stay(impl):
+    """Under the tail filter the update creates an entry and writes its sector back: every key is there once afterwards."""
+    from parameter_server_b200.models.ftrl import DeviceMinibatch, FTRLEngine, FTRLHyper
+    from parameter_server_b200.parallel.peer import PeerGroup
+
+    hyper = FTRLHyper(alpha=0.1, beta=1.0, lambda1=0.0, lambda2=0.1, rule="count", tail_feature_freq=1, countmin_n=1 << 24)
+    n = 60_000
+    eng = FTRLEngine(PeerGroup.single(torch.device("cuda", 0)), hyper, table_capacity=1 << 18, max_rows=4096, max_nnz=2 * n, local_capacity=1 << 18,
+                     impl=impl)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    keys = torch.arange(1, n + 1, device="cuda") * 0x9E3779B97F4A7C15
+    off = torch.arange(0, 2 * n + 1, 40, device="cuda")
+    for _ in range(3):
+        mb = torch.cat([keys, keys])[torch.randperm(2 * n, generator=g, device="cuda")]      # every key passes the filter at once
+        eng.step(DeviceMinibatch(off, mb, torch.ones(off.numel() - 1, device="cuda")))
+        eng.check_status()
+        held = eng.tab.local[:, 0]
+        assert torch.equal(held[held != -1].sort().values, keys.sort().values)
+    assert eng.read_stats(reset=False)["table_entries"] == n
+
+
 def test_model_text_dump(tmp_path):
     from parameter_server_b200.models.ftrl import DeviceMinibatch
     from parameter_server_b200.utils.modelio import read_model_text
