@@ -1169,9 +1169,9 @@ int psb_ftrl_pull_spmv(const FtrlPeers* P, const Minibatch* M, const LocalScratc
 constexpr int64_t kTwoLaunchNnz = 1500000;
 
 // One training step: pull, rows, push (sequence numbers of the pull's and the push's flags).  flags bit 0: create
-// missing keys in the shard.
+// missing keys in the shard.  launches: the kernels launched are added.
 int psb_ftrl_step(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L, const FtrlHyper* H, uint32_t pull_seq,
-                  uint32_t push_seq, uint32_t flags, cudaStream_t stream) {
+                  uint32_t push_seq, uint32_t flags, int* launches, cudaStream_t stream) {
   const bool soa = L->soa != 0;
   const bool filter = H->tail_freq != 0u && H->cm != nullptr;
   if (L->lt_w == nullptr || L->lt_acc == nullptr || P->in_slot == nullptr || L->region == nullptr) return (int)cudaErrorInvalidValue;
@@ -1182,6 +1182,7 @@ int psb_ftrl_step(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L,
   if (two) {
     const int e = launch_pull(P, M, L, pull_seq, flags & kPullInsert, stream);
     if (e != 0) return e;
+    ++*launches;
   }
   const void* kernels[4] = {(const void*)ftrl_step_kernel<false, false>, (const void*)ftrl_step_kernel<true, false>,
                             (const void*)ftrl_step_kernel<false, true>, (const void*)ftrl_step_kernel<true, true>};
@@ -1192,6 +1193,7 @@ int psb_ftrl_step(const FtrlPeers* P, const Minibatch* M, const LocalScratch* L,
   const int grid = step_grid(*P, *M, full, try_log2);
   FtrlPeers p = *P; Minibatch m = *M; LocalScratch l = *L; FtrlHyper h = *H;
   void* args[] = {&p, &m, &l, &h, &pull_seq, &push_seq, &flags, &try_log2};
+  ++*launches;
   return (int)cudaLaunchCooperativeKernel(kernels[which], dim3(grid), dim3(256), args, 0, stream);
 }
 

@@ -286,9 +286,10 @@ class FTRLEngine:
         self._L.parity = self.push_seq & 1 if self.group.world > 1 else 0
         # under the tail filter a key gets its entry only when it passes the filter, in the push
         insert = 1 if self.hyper.tail_feature_freq <= 0 else 0
+        launches = C.c_int(0)
         N.check(self._lib.psb_ftrl_step(C.byref(self._P), C.byref(M), C.byref(self._L), C.byref(self._H), C.c_uint32(self.pull_seq),
-                                        C.c_uint32(self.push_seq), C.c_uint32(insert), N.stream_ptr()), "ftrl_step")
-        self.kernel_launches += 1
+                                        C.c_uint32(self.push_seq), C.c_uint32(insert), C.byref(launches), N.stream_ptr()), "ftrl_step")
+        self.kernel_launches += launches.value
 
     def predict(self, mb: DeviceMinibatch) -> torch.Tensor:
         """X·w for a minibatch with the current model (collective: every rank calls it between steps).

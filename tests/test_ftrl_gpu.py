@@ -203,6 +203,21 @@ def test_keys_entered_by_the_update_itself_stay(impl):
     assert eng.read_stats(reset=False)["table_entries"] == n
 
 
+@pytest.mark.parametrize("threshold,launches", [(1, 2), (1 << 60, 1)])
+def test_launches_of_a_step_are_counted(threshold, launches):
+    from parameter_server_b200.models.ftrl import DeviceMinibatch
+
+    eng, _ = _engine()
+    eng._L.two_launch_nnz = threshold
+    mb = DeviceMinibatch(*_batches(1)[0])
+    before = eng.kernel_launches
+    for _ in range(3):
+        eng.step(mb)
+    assert eng.kernel_launches - before == 3 * launches
+    eng.predict(mb)
+    assert eng.kernel_launches - before == 3 * launches + 1
+
+
 def test_model_text_dump(tmp_path):
     from parameter_server_b200.models.ftrl import DeviceMinibatch
     from parameter_server_b200.utils.modelio import read_model_text
