@@ -179,7 +179,7 @@ __device__ __forceinline__ size_t acc_bytes() { return kCounts ? sizeof(AccSlot)
 #define PSB_ST_U32(p, v, pol) st_stream_u32((p), (v), (pol))
 
 // trace slots: 0 start, 1 localized, 2 all owners replied, 3 rows done (a step: gradients too),
-//              4 flags sent and tables cleared, 5 applied
+//              4 flags sent and tables cleared, 5 applied; of two launches 6 the start of the second
 #define PSB_TRACE(L, gtid, i) do { if ((L).trace != nullptr && (gtid) == 0) (L).trace[i] = globaltimer_ns(); } while (0)
 
 // Both tables index with the TOP bits of the same 64-bit hash (see FtrlPeers).
@@ -930,6 +930,7 @@ ftrl_step_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t
     rlog2 = pull_weights<2>(grid, P, M, L, pull_seq, flags, try_log2, gtid, gsz, &sh_ok);
   } else {
     rlog2 = __ldcg(L.region + kRegionNow);
+    PSB_TRACE(L, gtid, 6);
   }
   phase_rows<kCounts>(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, lane, &hot);
   if (world > 1) __threadfence_system();   // the accumulators must be visible to their owners before the flag is

@@ -195,6 +195,7 @@ class FTRLEngine:
             self._H.cm_k, self._H.tail_freq = max(int(hyper.countmin_k), 1), int(hyper.tail_feature_freq)
         self._lib = N.lib()
         self.kernel_launches = 0
+        self._step_launches = 1     # of the last step
         self.grown = 0
         if impl == "nccl":
             self._u_keys = torch.empty((self.lcap,), dtype=i64, device=d)
@@ -289,6 +290,7 @@ class FTRLEngine:
         launches = C.c_int(0)
         N.check(self._lib.psb_ftrl_step(C.byref(self._P), C.byref(M), C.byref(self._L), C.byref(self._H), C.c_uint32(self.pull_seq),
                                         C.c_uint32(self.push_seq), C.c_uint32(insert), C.byref(launches), N.stream_ptr()), "ftrl_step")
+        self._step_launches = launches.value
         self.kernel_launches += launches.value
 
     def predict(self, mb: DeviceMinibatch) -> torch.Tensor:
@@ -403,11 +405,12 @@ class FTRLEngine:
 
     def phase_times_us(self) -> dict:
         """Durations (µs) of the phases of the last fused step, from in-kernel globaltimer marks; "rows" is X·w, the
-        loss and the gradients."""
+        loss and the gradients, "kernel_gap" the time between the two launches of a large step."""
         t = self.trace.tolist()
         d = lambda a, b: (t[b] - t[a]) / 1e3
-        return {"localize": d(0, 1), "lookup_reply": d(1, 2), "rows": d(2, 3), "flag_reset": d(3, 4), "apply": d(4, 5),
-                "step": d(0, 5)}
+        rows = 6 if self._step_launches == 2 else 2
+        return {"localize": d(0, 1), "lookup_reply": d(1, 2), "kernel_gap": d(2, rows), "rows": d(rows, 3), "flag_reset": d(3, 4),
+                "apply": d(4, 5), "step": d(0, 5)}
 
     def penalty(self, st: dict) -> float:
         """λ₁‖w‖₁ + ½λ₂·sqrt(‖w‖₂²) exactly as FTRLModel::objv (src/linear_method/ftrl_model.h:31)."""

@@ -218,6 +218,21 @@ def test_launches_of_a_step_are_counted(threshold, launches):
     assert eng.kernel_launches - before == 3 * launches + 1
 
 
+@pytest.mark.parametrize("threshold", [1, 1 << 60])
+def test_phase_times_tell_the_gap_between_two_launches(threshold):
+    from parameter_server_b200.models.ftrl import DeviceMinibatch
+
+    eng, _ = _engine()
+    eng._L.two_launch_nnz = threshold
+    mb = DeviceMinibatch(*_batches(1)[0])
+    for _ in range(3):
+        eng.step(mb)
+    t = eng.phase_times_us()
+    assert all(v >= 0 for v in t.values()) and t["rows"] > 0
+    assert sum(v for k, v in t.items() if k != "step") == pytest.approx(t["step"], abs=0.01)
+    assert t["kernel_gap"] > 0 if threshold == 1 else t["kernel_gap"] == 0
+
+
 def test_model_text_dump(tmp_path):
     from parameter_server_b200.models.ftrl import DeviceMinibatch
     from parameter_server_b200.utils.modelio import read_model_text
