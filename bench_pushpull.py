@@ -8,8 +8,9 @@ Key sets of n uint64 keys (Zipf(1.1) over a 2^32 key space, de-duplicated) with 
   * the same two operations with ``all_to_all_single`` + local gather / scatter-add kernels
 and, with ``--fused``, the fused FTRL step on a minibatch whose n non-zeros are n distinct keys (32 per
 row, value length 1): its pull (de-duplication, lookup, weights back) and its rows and push (X·w, gradient,
-FTRL update), told apart by the marks inside the kernels, against the NCCL-only engine's pull and push of
-the same minibatch.  It reports GB/s of payload per GPU and the fraction of the NVLink roofline
+FTRL update) against the NCCL-only engine's pull and push of the same minibatch.  Both arms are timed with
+CUDA events around the whole step; the fused step's time is split in the proportion of the marks inside its
+kernels.  It reports GB/s of payload per GPU and the fraction of the NVLink roofline
 (bytes that must cross NVLink / 770 GB/s measured peer-copy bandwidth per direction per GPU); for the
 fused kernels the payload is 12 bytes per key for the pull (key out, weight back) and 4 bytes for the
 push (gradient), and small key sets are reported as latency.
@@ -29,6 +30,13 @@ if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
 NVLINK_GBS = 770.0
+
+
+def split_step(ms: float, phases: dict):
+    """(pull, push) of a fused step that took ``ms`` between two events, in the proportion of its in-kernel marks; what
+    the marks do not see (the launches, the tail of the other thread blocks) is shared out with it."""
+    pull = (phases["localize"] + phases["lookup_reply"]) / max(phases["step"], 1e-9)
+    return ms * pull, ms * (1.0 - pull)
 
 
 def main() -> None:
@@ -83,26 +91,27 @@ def main() -> None:
             ev = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
             t_pull = t_push = 0.0
             for it in range(args.warmup + iters):
+                ev[0].record()
                 if impl == "fused":
-                    eng.step(mb)     # one kernel; its own marks tell the pull from the rows and the push
+                    eng.step(mb)
                 else:
-                    M = eng._mb(mb)
-                    ev[0].record()
-                    ctx = eng._pull_nccl(M)
+                    ctx = eng._pull_nccl(eng._mb(mb))
                     ev[1].record()
-                    eng._push_nccl(M, *ctx)
-                    ev[2].record()
+                    eng._push_nccl(eng._mb(mb), *ctx)
+                ev[2].record()
                 torch.cuda.synchronize(dev)
-                if it >= args.warmup and impl == "fused":
-                    ph = eng.phase_times_us()
-                    t_pull += (ph["localize"] + ph["lookup_reply"]) / 1e3
-                    t_push += (ph["rows"] + ph["flag_reset"] + ph["apply"]) / 1e3
-                elif it >= args.warmup:
-                    t_pull += ev[0].elapsed_time(ev[1])
-                    t_push += ev[1].elapsed_time(ev[2])
+                if it < args.warmup:
+                    continue
+                if impl == "fused":
+                    pull, push = split_step(ev[0].elapsed_time(ev[2]), eng.phase_times_us())
+                else:
+                    pull, push = ev[0].elapsed_time(ev[1]), ev[1].elapsed_time(ev[2])
+                t_pull += pull
+                t_push += push
             eng.check_status()
             ms_pull = group.all_reduce_max(t_pull / iters)
             ms_push = group.all_reduce_max(t_push / iters)
+            row[f"{impl}_step_us"] = group.all_reduce_max((t_pull + t_push) / iters) * 1e3
             remote = (W - 1) / max(W, 1)
             for name, ms, bytes_per_key in (("pull", ms_pull, 12), ("push", ms_push, 4)):
                 row[f"{impl}_{name}_us"] = ms * 1e3

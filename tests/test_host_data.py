@@ -143,3 +143,12 @@ def test_columns_from_rows_refuses_values_and_offsets_that_do_not_belong_to_the_
         sparse.columns_from_rows(off.to("meta"), keys, torch.ones(4))
     with pytest.raises(ValueError, match="3 values for 4"):
         sparse.columns_from_rows(off.to("meta"), keys, torch.ones(3, device="meta"))
+
+
+def test_pushpull_benchmark_splits_the_whole_step():
+    """The two parts of the fused step add up to what the events around it measured, as those of the other arm do."""
+    import bench_pushpull
+
+    pull, push = bench_pushpull.split_step(2.0, {"localize": 100.0, "lookup_reply": 50.0, "kernel_gap": 10.0, "rows": 90.0, "flag_reset": 5.0,
+                                                 "apply": 45.0, "step": 300.0})
+    assert pull == pytest.approx(1.0) and pull + push == pytest.approx(2.0)
