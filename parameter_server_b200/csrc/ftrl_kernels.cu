@@ -410,7 +410,6 @@ __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScra
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
         const uint32_t i = (uint32_t)(k + j) * 256u + threadIdx.x;
-        if (i >= chunk) continue;
         uint32_t slot = kBadSlot;
         float w = 0.f;
         if (key[k + j] != kEmptyKey) {
@@ -424,6 +423,10 @@ __device__ __forceinline__ void phase_lookup(const FtrlPeers& P, const LocalScra
             slot = kAhead > 1 && hk[j] == kEmptyKey ? kAbsent : shard_find(P.tab, P.tab_mask, P.tab_shift, key[k + j], P.max_probe, &w);
           }
         }
+        // Lanes leave the probes above at different times.  Without the meeting point a warp stores in pieces, and parts
+        // of sectors are slow: 9.6 M distinct keys in 2^24 slots, lookup 312 -> 217 us.
+        __syncwarp();
+        if (i >= chunk) continue;
         P.in_slot[in0 + i] = slot;
         if (P.in_keys != nullptr) P.in_keys[in0 + i] = key[k + j];
         if (have_ok) {
