@@ -69,3 +69,11 @@ def test_resolve_over_list_orders_and_run_lengths(n, shards, held):
             hit[hit] = keep[r][0][at[hit]] == query[hit]
             want[hit] = at[hit]
         assert np.array_equal(owner.cpu().numpy(), o) and np.array_equal(slot.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n,held", [(151_551, 60_000), (151_552, 400_000), (151_553, 60_000), (303_103, 60_000), (303_104, 1_000_000),
+                                    (303_105, 60_000), (2_600_000, 4_000_000)])
+@pytest.mark.parametrize("shards", [1, 3])
+def test_resolve_with_several_queries_a_thread(n, shards, held):
+    """Two and four queries a thread (from 151,552 and 303,104 on), and more tiles than the grid has thread blocks."""
+    test_resolve_over_list_orders_and_run_lengths(n, shards, held)
