@@ -10,8 +10,8 @@
 //                      ("empty" mbarrier) and finally signals "accumulator complete"
 //   all 4 warps        epilogue: tcgen05.ld 32 lanes x 32 columns per warp and step, activation, store
 // Both operands are K-major (row-major with K contiguous), which is how the layers keep their data:
-// activations [batch, features] and weights [out, in]; the transposed products of the backward
-// pass go through the tiled transpose kernel first.  No multicast is used anywhere.
+// activations [batch, features] and weights [out, in]; the products of the backward pass read transposes that
+// an epilogue, the activation's slope or the tiled transpose kernel wrote.  No load is a multicast.
 //
 // This is the framework's replacement of the Eigen GEMMs of the reference's fully connected
 // layer (src/neural_network/fully_connected_layer.h:27-65); the activation functions are those
@@ -638,7 +638,7 @@ EncodeTiledFn get_encode() {
   }
   return fn;
 }
-// 2-D map over a row-major [rows, k] fp32 matrix with row stride ld (floats), box = 128 rows x 32 floats, 128B swizzle
+// 2-D map over a row-major [rows, k] fp32 matrix with row stride ld (floats), box = box_rows rows x 32 floats, 128B swizzle
 int make_map(CUtensorMap* map, const float* base, int rows, int k, int ld, int box_rows) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return -1;

@@ -11,8 +11,8 @@ ranks train data-parallel: every rank draws its own minibatches and the weight g
 all-reduced over NCCL before the update.
 
 Layout: activations are ``[batch, features]``, weights are stored ``[out, in]`` so that both GEMM
-operands of the forward pass are K-major; the two products of the backward pass get their
-operands from the tiled transpose kernel.  ``scaled tanh`` is 1.7159·tanh(⅔·x) — the reference
+operands of the forward pass are K-major; the two products of the backward pass read transposes
+that the forward GEMM, the activation's slope or the transpose kernel wrote.  ``scaled tanh`` is 1.7159·tanh(⅔·x) — the reference
 writes ``2/3`` in integer arithmetic, which evaluates to 0; the documented formula is used.
 """
 from __future__ import annotations
