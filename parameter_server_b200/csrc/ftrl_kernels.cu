@@ -157,7 +157,7 @@ struct LocalScratch {
 // How much of the per-minibatch table a step uses.  The table is allocated for the largest minibatch the job may
 // send, but every slot of it is walked four times a step (owner lookup, owner update, key reset, accumulator
 // reset) and its keys and accumulators are probed at random, so a step works in the first 2^r slots only: r from
-// the minibatch's non-zeros (psb_ftrl_pull_spmv's `try_log2`), twice the slots as often as its keys do not fit.
+// the minibatch's non-zeros (first_region_log2), twice the slots as often as its keys do not fit (phase_localize).
 // One GPU only: with several, chunk c of every worker's table must cover the same key range.
 // B200, 10,000 rows (0.34 M keys) with the tail filter in 2^22 / 2^20 slots: step 264 / 167 us before the other changes;
 // 100,000 rows (2.4 M keys) in 2^24 / 2^22: 825 / 699 us.
@@ -250,8 +250,12 @@ __device__ __forceinline__ uint64_t place_key(uint64_t* keys, uint64_t cmask, ui
 }
 
 // Returns the number of keys this thread entered.  With fewer than 2^P.region_log2 slots a key that finds no
-// place leaves the size in the misfit word instead of an error, and the thread gives up: the caller starts over with
-// more slots.
+// place within kFullChain slots leaves the size in the misfit word instead of an error, and its block gives up: the
+// caller starts over with more slots.  So long a chain comes up when about 0.7 of a large table is taken, and from
+// there on a new key walks dozens of slots, one dependent read each.  B200, 9.6 M non-zeros, sum of squares, in 2^22 /
+// 2^23 / 2^24 slots: 2.9 M keys (0.69 of the smallest) 611 / 553 / 697 us a step, 3.2 M 680 / 575 / 707, 3.5 M 806 / 594 / 728.
+// The step that finds out takes 0.3 to 1 ms more, once for an engine.
+constexpr int kFullChain = 256;
 __device__ __forceinline__ uint32_t phase_localize(const FtrlPeers& P, const Minibatch& M, const LocalScratch& L,
                                                    size_t gtid, size_t gsz, uint32_t rlog2) {
   PSB_STREAM_POLICY(pol);
@@ -259,6 +263,10 @@ __device__ __forceinline__ uint32_t phase_localize(const FtrlPeers& P, const Min
   const uint64_t region = 1ull << rlog2;
   const uint64_t cmask = (region < (uint64_t)kChunkSlots ? region : (uint64_t)kChunkSlots) - 1;
   const Refs refs(P, rlog2);
+  const int max_probe = rlog2 < P.region_log2 && kFullChain < P.max_probe ? kFullChain : P.max_probe;
+  __shared__ int s_full;
+  if (threadIdx.x == 0) s_full = 0;
+  __syncthreads();
   uint32_t fresh = 0;
   int64_t i = (int64_t)gtid;
   if (i >= M.nnz) return 0u;
@@ -273,9 +281,10 @@ __device__ __forceinline__ uint32_t phase_localize(const FtrlPeers& P, const Min
       h1 = local_home(P, key1, rlog2);
       cur1 = ld_table_u64(L.lt_keys + (uint32_t)h1);
     }
-    const uint64_t at = place_key(L.lt_keys, cmask, (uint32_t)h0, key0, P.max_probe, cur0, &fresh);
+    const uint64_t at = place_key(L.lt_keys, cmask, (uint32_t)h0, key0, max_probe, cur0, &fresh);
+    if (*(volatile int*)&s_full) break;
     if (at == ~0ull) {
-      if (rlog2 < P.region_log2) { L.region[kRegionMisfit] = rlog2; break; }
+      if (rlog2 < P.region_log2) { L.region[kRegionMisfit] = rlog2; s_full = 1; break; }
       set_status(L.status, kLocalTableFull, 0, 0);
     }
     PSB_ST_U32(L.slot_of + i, refs.make((uint32_t)at, (uint32_t)(h0 >> 32)), pol);      // (uint32_t)~0 is kBadSlot

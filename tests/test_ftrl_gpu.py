@@ -233,6 +233,33 @@ def test_phase_times_tell_the_gap_between_two_launches(threshold):
     assert t["kernel_gap"] > 0 if threshold == 1 else t["kernel_gap"] == 0
 
 
+@pytest.mark.parametrize("rule", ["count", "sumsq"])
+@pytest.mark.parametrize("share,log2", [(0.5, 18), (0.75, 19), (0.87, 19)])
+def test_a_table_with_long_chains_is_left_for_a_larger_one(rule, share, log2):
+    """300,000 non-zeros start in 2^18 slots; keys that would fill them to 0.86 fit, but at the end of long chains."""
+    from parameter_server_b200.models.ftrl import DeviceMinibatch
+
+    eng, hy = _engine(rule=rule, table_capacity=1 << 21, local_capacity=1 << 20, max_rows=8192)
+    ref = FTRLRef(hy.alpha, hy.beta, hy.lambda1, hy.lambda2, rule)
+    g = torch.Generator(device="cuda").manual_seed(6)
+    n = 300_000
+    for _ in range(2):
+        ids = torch.cat([torch.arange(int(n * share), device="cuda"),
+                         torch.randint(0, int(n * share), (n - int(n * share),), generator=g, device="cuda")])
+        keys = ids[torch.randperm(n, generator=g, device="cuda")] * 0x9E3779B9
+        off = torch.arange(0, n + 1, 60, device="cuda")
+        y = torch.where(torch.rand(n // 60, generator=g, device="cuda") < 0.5, 1.0, -1.0)
+        eng.step(DeviceMinibatch(off, keys, y))
+        eng.check_status()
+        assert int(eng.region[0].item()) == log2
+        ref.step([(off.cpu().numpy(), keys.cpu().numpy().view(np.uint64), y.cpu().numpy().astype(np.float64))])
+    k, w = eng.dump_model()
+    rk, rw = ref.nonzero()
+    assert np.array_equal(k, rk)
+    np.testing.assert_allclose(w, rw, rtol=2e-3, atol=2e-5)
+    assert eng.read_stats(reset=False)["table_entries"] == len(ref.model) == int(n * share)
+
+
 def test_model_text_dump(tmp_path):
     from parameter_server_b200.models.ftrl import DeviceMinibatch
     from parameter_server_b200.utils.modelio import read_model_text
