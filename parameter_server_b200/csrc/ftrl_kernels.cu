@@ -930,6 +930,11 @@ ftrl_pull_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_
 // 3 / 4 / 5 / 6 blocks per SM take 657 / 639 / 656 / 676 us a step (count rule), 690 / 580 / 590 / 600 (sum of squares);
 // from 5 on registers spill, with 3 too few random accesses are in flight.  Whole, 4 and 5 measure the same.
 constexpr int kStepBlocksPerSM = 5, kPushBlocksPerSM = 4;
+// Slots from which on the rows are walked twice, weights first, gradients then, when the table is larger than the
+// non-zeros alone ask for, that is when almost every slot is used: weights (64 MB) and accumulators fit the L2 one after
+// the other, not together.  9.6 M non-zeros in 2^24 slots, one walk / two: 9.6 M keys 1174 / 1136 us a step (sum of
+// squares) and 1444 / 1396 (count), 8.2 M 1065 / 1043 and 1305 / 1291, 6.7 M 944 / 945; 2.4 M 639 / 698.
+constexpr uint32_t kTwoWalksLog2 = 24;
 template <bool kCounts, bool kPull>
 __global__ void __launch_bounds__(256, kPull ? kStepBlocksPerSM : kPushBlocksPerSM)
 ftrl_step_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t pull_seq, uint32_t push_seq, uint32_t flags,
@@ -951,7 +956,13 @@ ftrl_step_kernel(FtrlPeers P, Minibatch M, LocalScratch L, FtrlHyper H, uint32_t
     rlog2 = __ldcg(L.region + kRegionNow);
     PSB_TRACE(L, gtid, 6);
   }
-  phase_rows<kCounts>(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, lane, &hot);
+  if (!kPull && world == 1 && rlog2 >= kTwoWalksLog2 && rlog2 > try_log2) {
+    phase_spmv_loss(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, lane, true);
+    grid.sync();
+    phase_grad<kCounts>(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, lane, &hot);
+  } else {
+    phase_rows<kCounts>(M, L, Refs(P, rlog2), gtid >> 5, gsz >> 5, lane, &hot);
+  }
   if (world > 1) __threadfence_system();   // the accumulators must be visible to their owners before the flag is
   grid.sync();
   PSB_TRACE(L, gtid, 3);

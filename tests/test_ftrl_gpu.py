@@ -260,6 +260,35 @@ def test_a_table_with_long_chains_is_left_for_a_larger_one(rule, share, log2):
     assert eng.read_stats(reset=False)["table_entries"] == len(ref.model) == int(n * share)
 
 
+@pytest.mark.parametrize("rule", ["count", "sumsq"])
+def test_millions_of_distinct_keys_match_the_unfused_engine(rule):
+    """Almost every slot of the largest table used: rows are walked once for the weights and once for the gradients."""
+    from parameter_server_b200.models.ftrl import DeviceMinibatch
+
+    n = 6_600_000
+    g = torch.Generator(device="cuda").manual_seed(9)
+    off = torch.arange(0, n + 1, 60, device="cuda")
+    y = torch.where(torch.rand(n // 60, generator=g, device="cuda") < 0.5, 1.0, -1.0)
+    mbs = [DeviceMinibatch(off, torch.randperm(n, generator=g, device="cuda") * 0x9E3779B97F, y) for _ in range(2)]
+    got = []
+    for impl in ("fused", "nccl"):
+        eng, _ = _engine(impl, rule, table_capacity=1 << 24, local_capacity=1 << 24, max_rows=n // 60, max_nnz=n)
+        for mb in mbs:
+            eng.step(mb)
+        eng.check_status()
+        if impl == "fused":
+            assert int(eng.region[0].item()) == 24
+        st = eng.read_stats(reset=False)
+        got.append((*eng.dump_model(), eng.predict(mbs[0]).cpu().numpy(), st["loss_sum"], st["table_entries"]))
+        del eng
+        torch.cuda.empty_cache()
+    (k, w, xw, loss, entries), (rk, rw, rxw, rloss, rentries) = got
+    assert entries == rentries == n and len(k) > 1000 and np.array_equal(k, rk)
+    np.testing.assert_allclose(w, rw, rtol=1e-4, atol=1e-6)
+    np.testing.assert_allclose(xw, rxw, rtol=1e-4, atol=1e-5)
+    assert loss == pytest.approx(rloss, rel=1e-6)
+
+
 def test_model_text_dump(tmp_path):
     from parameter_server_b200.models.ftrl import DeviceMinibatch
     from parameter_server_b200.utils.modelio import read_model_text
