@@ -810,13 +810,10 @@ class DarlinSolver:
 def repeat_in_group(order, group: int) -> int:
     """Position of the first block of ``order`` that its group of ``group`` consecutive entries holds already (0: none).
     A group that ends there is a shorter delay, which the bound allows."""
-    order = np.asarray(order)
-    if len(order) < 2 or np.bincount(order).max() < 2:
+    order = np.asarray(order).tolist()
+    if len(set(order)) == len(order):
         return 0
-    for i in range(1, len(order)):
-        if order[i] in order[i // group * group: i]:
-            return i
-    return 0
+    return next((i for i in range(1, len(order)) if order[i] in order[i // group * group: i]), 0)
 
 
 def print_progress(it: int, p: Progress, file=sys.stderr, busy=None) -> None:

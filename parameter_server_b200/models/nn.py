@@ -132,8 +132,9 @@ class DataLayer(Layer):
             b -= b % 4        # GEMM operand strides are multiples of 4 floats
             sel = torch.randperm(n, generator=self.gen)[:b].to(self.net.device)
             if dense.can_gather_minibatch(self.X, self.y, b):
-                xb, xbt, yb = dense.gather_minibatch(self.X, self.y, sel, self.net.keeps_transpose(self.outputs[0], b * self.X.shape[1]))
-                self.outputs[0].keep_transpose(xb, xbt)
+                out = self.outputs[0]
+                xb, xbt, yb = dense.gather_rows(self.X, self.y, sel, self.net.wants_transpose(out, b * self.X.shape[1]))
+                out.transposed = None if xbt is None else (xb, xb._version, xbt)
             else:
                 xb, yb = self.X[sel].contiguous(), self.y[sel].contiguous()
         self.outputs[0].value = xb
@@ -177,9 +178,9 @@ class FullyConnectedLayer(Layer):
         out = self.outputs[0]
         # a dense layer that reads this edge needs its transpose for the weight gradient: the GEMM writes both
         yt = torch.empty((self.out_dim, x.shape[0]), dtype=torch.float32, device=x.device) \
-            if self.net.keeps_transpose(out, x.shape[0] * self.out_dim) else None
+            if self.net.wants_transpose(out, x.shape[0] * self.out_dim) else None
         out.value = dense.gemm_tn(x, self.model.value, self.act, pad_k=True, out_t=yt)
-        out.keep_transpose(out.value, yt)
+        out.transposed = None if yt is None else (out.value, out.value._version, yt)
         return 0.0
 
     def backward(self) -> None:
@@ -188,7 +189,7 @@ class FullyConnectedLayer(Layer):
             z, zt = gy, _transposed(gy)
         else:
             z, zt = dense.act_backward_t(gy, y, self.act, want_z=self.inputs[0].needs_grad)
-        xt = self.inputs[0].take_transpose(self.x)
+        xt = self.net.take_transpose(self.inputs[0], self.x)
         xt = _transposed(self.x) if xt is None else xt
         self.model.gradient = dense.gemm_tn(zt, xt, pad_k=True)                       # [out, in] = Zᵀ · X
         if self.inputs[0].needs_grad:
@@ -261,16 +262,6 @@ class Edge(Parameter):
     read_by_dense: bool = False                  # a fully connected layer has this edge as its input
     transposed: Optional[tuple] = None           # (value, its version, valueᵀ) from the layer that wrote the value
 
-    def keep_transpose(self, value: torch.Tensor, t: Optional[torch.Tensor]) -> None:
-        """``t`` is ``valueᵀ`` (None: it is not at hand) until the value is written to.  A tensor of inference mode does
-        not tell when it was written to, and its transpose is not kept."""
-        self.transposed = None if t is None or value.is_inference() else (value, value._version, t)
-
-    def take_transpose(self, value: torch.Tensor) -> Optional[torch.Tensor]:
-        """The kept transpose of ``value`` if it still is that; it is not kept any longer."""
-        t, self.transposed = self.transposed, None
-        return t[2] if t is not None and t[0] is value and value._version == t[1] else None
-
 
 # Transposes that a net's forward pass writes along and keeps for its backward pass, in bytes.  Without a bound a
 # full-batch net held every activation twice, where one transpose at a time lives in the backward pass otherwise; 0.3 %
@@ -284,6 +275,7 @@ class Net:
     def __init__(self, conf, group: PeerGroup, shared_models: Optional[Dict[str, Parameter]] = None, training: bool = True):
         self.conf, self.group, self.device, self.training = conf, group, group.device, training
         self.edges: Dict[str, Edge] = {}
+        self.kept_bytes = 0                      # of the edges' transposes
         self.shared_models = shared_models if shared_models is not None else {}
         self.layers: List[Layer] = []
         for lc in conf.layer:
@@ -303,14 +295,29 @@ class Net:
             self.edges[name] = Edge(name)
         return self.edges[name]
 
-    def keeps_transpose(self, edge: Edge, numel: int) -> bool:
-        """Whether the layer that writes ``numel`` elements to ``edge`` writes their transpose too, for the weight
-        gradient of the dense layer that reads it.  What is kept until the backward pass stays below a bound."""
-        edge.transposed = None
-        if not self.training or not edge.read_by_dense or torch.is_inference_mode_enabled():
+    def wants_transpose(self, edge: Edge, numel: int) -> bool:
+        """Whether the layer that writes ``numel`` elements to ``edge`` is to write their transpose too, for the weight
+        gradient of the dense layer that reads it.  What is kept until the backward pass stays below a bound, and a tensor
+        of inference mode cannot tell whether it was written to since."""
+        if edge.transposed is not None:
+            self._drop_transpose(edge)
+        if not self.training or not edge.read_by_dense or torch.is_inference_mode_enabled() \
+                or self.kept_bytes + 4 * numel > KEPT_TRANSPOSE_BYTES:
             return False
-        kept = sum(e.transposed[2].nbytes for e in self.edges.values() if e.transposed is not None)
-        return kept + 4 * numel <= KEPT_TRANSPOSE_BYTES
+        self.kept_bytes += 4 * numel
+        return True
+
+    def take_transpose(self, edge: Edge, value: torch.Tensor) -> Optional[torch.Tensor]:
+        """The kept transpose of ``value`` if it still is that; it is not kept any longer."""
+        t = edge.transposed
+        if t is None:
+            return None
+        self._drop_transpose(edge)
+        return t[2] if t[0] is value and value._version == t[1] else None
+
+    def _drop_transpose(self, edge: Edge) -> None:
+        self.kept_bytes -= 4 * edge.transposed[2].numel()
+        edge.transposed = None
 
     def layer(self, name: str) -> Layer:
         return next(l for l in self.layers if l.name == name)

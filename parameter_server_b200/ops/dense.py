@@ -81,7 +81,7 @@ def act_backward(g: torch.Tensor, y: torch.Tensor, act: str) -> torch.Tensor:
 def act_backward_t(g: torch.Tensor, y: torch.Tensor, act: str, want_z: bool = True):
     """(``g ∘ act'(y)`` or None, its transpose) of two contiguous [rows, cols] matrices in one pass over them."""
     assert g.is_contiguous() and y.is_contiguous() and g.shape == y.shape and g.dim() == 2
-    assert g.is_cuda and g.device == y.device and g.dtype == y.dtype == torch.float32
+    assert g.is_cuda and y.is_cuda and g.dtype == y.dtype == torch.float32
     z = torch.empty_like(g) if want_z else None
     zt = torch.empty((g.shape[1], g.shape[0]), dtype=torch.float32, device=g.device)
     N.check(N.lib().psb_act_backward_t(N.ptr(g), N.ptr(y), N.ptr(z), N.ptr(zt), g.shape[0], g.shape[1], ACT[act], N.stream_ptr()),
@@ -89,16 +89,21 @@ def act_backward_t(g: torch.Tensor, y: torch.Tensor, act: str, want_z: bool = Tr
     return z, zt
 
 
-def can_gather_minibatch(x: torch.Tensor, y: torch.Tensor, b: int) -> bool:
-    """The data that :func:`gather_minibatch` takes: one label per row (labels of several columns are indexed)."""
-    return (x.is_cuda and x.device == y.device and x.dtype == y.dtype == torch.float32 and x.dim() == 2 and y.shape == x.shape[:1]
-            and x.shape[1] > 0 and x.is_contiguous() and y.is_contiguous() and 0 < b <= 32 * 65535)
-
-
 def gather_minibatch(x: torch.Tensor, y: torch.Tensor, sel: torch.Tensor, want_t: bool):
     """(``x[sel]``, its transpose or None, ``y[sel]``) for contiguous float32 ``x`` [n, cols], ``y`` [n] and device
     int64 row numbers ``sel`` (all inside x), in one launch."""
-    assert can_gather_minibatch(x, y, sel.numel()) and sel.device == x.device and sel.is_contiguous() and sel.dtype == torch.int64
+    assert can_gather_minibatch(x, y, sel.numel()) and sel.is_cuda and sel.is_contiguous() and sel.dtype == torch.int64
+    return gather_rows(x, y, sel, want_t)
+
+
+def can_gather_minibatch(x: torch.Tensor, y: torch.Tensor, b: int) -> bool:
+    """The data that :func:`gather_minibatch` takes: one label per row (labels of several columns are indexed)."""
+    return (x.is_cuda and y.is_cuda and x.dtype == y.dtype == torch.float32 and x.dim() == 2 and y.dim() == 1
+            and y.numel() == x.shape[0] and x.numel() > 0 and x.is_contiguous() and y.is_contiguous() and 0 < b <= 32 * 65535)
+
+
+def gather_rows(x: torch.Tensor, y: torch.Tensor, sel: torch.Tensor, want_t: bool):
+    """:func:`gather_minibatch` of data that was found fit for it."""
     b, cols = sel.numel(), x.shape[1]
     xb = torch.empty((b, cols), dtype=torch.float32, device=x.device)
     yb = torch.empty(b, dtype=torch.float32, device=x.device)

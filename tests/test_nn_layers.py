@@ -82,7 +82,7 @@ def test_gradients(ops):
     sol.train.forward()
     sol.train.backward()
     _check_gradients(sol, X, y)
-    assert len(ops) == 2 and all(e.transposed is None for e in sol.train.edges.values())
+    assert len(ops) == 2 and all(e.transposed is None for e in sol.train.edges.values()) and sol.train.kept_bytes == 0
 
 
 @pytest.mark.parametrize("offset", [0, 1, 2, 3])
