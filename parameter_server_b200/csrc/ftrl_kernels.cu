@@ -907,7 +907,8 @@ __device__ __forceinline__ uint32_t pull_weights(cg::grid_group& grid, const Ftr
 // The pull on its own: of a large training step, and of a prediction, which also multiplies the rows, empties the
 // key table again (every owner has replied, nobody reads it any more) and leaves the statistics alone: one launch
 // where saving and restoring them and emptying the table took four more.  8 blocks of 256 threads per SM (32
-// registers per thread): its phases are bound by memory latency and speed up with every resident warp.
+// registers per thread, 24 bytes spilled): its phases are bound by memory latency.  9.6 M non-zeros of 2.4 M keys take
+// the same time with 6 blocks and no spills, and with the prediction compiled apart.
 constexpr int kPullBlocksPerSM = 8;
 __global__ void __launch_bounds__(256, kPullBlocksPerSM)
 ftrl_pull_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_t flags, uint32_t try_log2) {
@@ -928,7 +929,8 @@ ftrl_pull_kernel(FtrlPeers P, Minibatch M, LocalScratch L, uint32_t seq, uint32_
 
 // A training step, whole (kPull) or after ftrl_pull_kernel: rows and push.  Rows and push alone: 100,000 rows with
 // 3 / 4 / 5 / 6 blocks per SM take 657 / 639 / 656 / 676 us a step (count rule), 690 / 580 / 590 / 600 (sum of squares);
-// from 5 on registers spill, with 3 too few random accesses are in flight.  Whole, 4 and 5 measure the same.
+// from 5 on registers spill (at 4, 16 bytes of the sum of squares), with 3 too few random accesses are in flight.  Whole, 4 and
+// 5 measure the same; 5 spills 36 to 68 bytes.
 constexpr int kStepBlocksPerSM = 5, kPushBlocksPerSM = 4;
 // Slots from which on the rows are walked twice, weights first, gradients then, when the table is larger than the
 // non-zeros alone ask for, that is when almost every slot is used: weights (64 MB) and accumulators fit the L2 one after
