@@ -810,7 +810,7 @@ class DarlinSolver:
 def repeat_in_group(order, group: int) -> int:
     """Position of the first block of ``order`` that its group of ``group`` consecutive entries holds already (0: none).
     A group that ends there is a shorter delay, which the bound allows."""
-    order = np.asarray(order).tolist()
+    order = order.tolist() if hasattr(order, "tolist") else list(order)      # an array, or a tensor on any device
     if len(set(order)) == len(order):
         return 0
     return next((i for i in range(1, len(order)) if order[i] in order[i // group * group: i]), 0)

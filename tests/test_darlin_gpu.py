@@ -158,7 +158,7 @@ def test_block_twice_in_one_bounded_delay_group(variant, wide):
         sol.pass_variant = variant
         sol.preprocess(off, keys, vals, y)
         for o in orders:
-            sol.launch_pass(np.asarray(o, dtype=np.int32))
+            sol.launch_pass(torch.tensor(o, dtype=torch.int32, device="cuda") if tau == 1 else np.asarray(o, dtype=np.int32))
         sol.check_status()
         want = margins_from_weights(sol.col_ptr, sol.row_idx, sol.vals, sol.y, sol.w)
         assert torch.allclose(sol.margin, want, rtol=1e-4, atol=1e-4)

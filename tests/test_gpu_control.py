@@ -256,9 +256,11 @@ def test_online_job_does_not_hang_when_a_rank_vanishes(tmp_path):
 
 def test_repeat_in_group():
     import numpy as np
+    import torch
 
     from parameter_server_b200.models.darlin import repeat_in_group
 
     for order, group, want in (([], 3, 0), ([2], 3, 0), ([0, 1, 2, 0], 3, 0), ([0, 1, 0, 2], 3, 2), ([5, 5], 2, 1), ([5, 5], 1, 0),
                                ([0, 1, 2, 3, 4, 3], 3, 5), ([0, 1, 2, 1, 0], 3, 0)):
-        assert repeat_in_group(np.asarray(order, dtype=np.int32), group) == want, order
+        for form in (np.asarray(order, dtype=np.int32), order, tuple(order), torch.tensor(order, dtype=torch.int32)):
+            assert repeat_in_group(form, group) == want, (order, type(form))
