@@ -597,11 +597,12 @@ class DarlinSolver:
             finally:
                 self.cfg.max_block_delay = saved
         if self.cfg.max_block_delay > 0 and self.group.world == 1 and self.impl == "fused" and not self.out_of_core:
-            cut = repeat_in_group(order, self.cfg.max_block_delay + 1)
+            group = min(int(self.cfg.max_block_delay) + 1, MAX_GROUP)
+            cut = repeat_in_group(order, group)
             while cut:       # two threads would step that block's columns
                 self.launch_pass(order[:cut], first=first)
                 order, first = order[cut:], False
-                cut = repeat_in_group(order, self.cfg.max_block_delay + 1)
+                cut = repeat_in_group(order, group)
         order_t = torch.as_tensor(order, dtype=torch.int32).to(self.dev, non_blocking=False)
         self._order_keepalive = order_t
         if first:
@@ -805,6 +806,9 @@ class DarlinSolver:
         path = f"{file_prefix}_S{self.group.rank}"
         write_model_text(path, k, w)
         return path
+
+
+MAX_GROUP = 128    # blocks that the pass kernel sweeps together at most (kMetaSlots / 4 in csrc/darlin_kernels.cu)
 
 
 def repeat_in_group(order, group: int) -> int:
